@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(Q_THREADS) quant_kernel(const __nv_bfloat16* _
         for (int e = 0; e < 8; ++e) { x[2 * e] = __uint_as_float(w[e] << 16); x[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u); }
         uint2 c;
         uint8_t sf;
-        qm::quant_block16(x, gs, rule, c, sf);
+        qm::quant_block16<false>(x, gs, rule, c, sf);
         const int r = row & 127, b16 = kb & 15, ch = b16 >> 1;
         uint8_t* out = rec + ((size_t)(row >> 7) * nkt + (kb >> 4)) * A_REC;
         *reinterpret_cast<uint2*>(out + r * 128 + ((ch ^ (r & 7)) << 4) + (b16 & 1) * 8) = c;

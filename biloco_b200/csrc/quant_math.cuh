@@ -126,12 +126,23 @@ __device__ __forceinline__ uint32_t codes8(const float* x, float d) {
 }
 __device__ __forceinline__ uint2 codes16(const float (&x)[16], float d) { return make_uint2(codes8(x, d), codes8(x + 8, d)); }
 
+// The larger of two values; NaN if either is (fmaxf drops it).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+
 // One thread, one block of sixteen values (the throughput form: thousands of blocks): the arithmetic of the file header.
+// KEEP_NAN (weights): a NaN makes the block's maximum and with it its scale NaN (0x7f, codes 0), and a tensor scale that is not
+// positive gives a scale of zero, as torch's maximum and clamp have it. Otherwise (activations) maxima drop NaN.
+template <bool KEEP_NAN>
 __device__ __forceinline__ void quant_block16(const float (&x)[16], float gs, int rule, uint2& codes, uint8_t& sf) {
     float bmax = 0.f;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) bmax = fmaxf(bmax, fabsf(x[j]));
-    const float t = __fdiv_rn(bmax, gs);
+    for (int j = 0; j < 16; ++j) bmax = KEEP_NAN ? max_nan(bmax, fabsf(x[j])) : fmaxf(bmax, fabsf(x[j]));
+    float t = __fdiv_rn(bmax, gs);
+    if (KEEP_NAN && t <= 0.f) t = 0.f;
     uint2 c[2];
     uint8_t s[2] = {0, 0};
     float e[2] = {0.f, 0.f};

@@ -20,9 +20,11 @@ namespace {
 constexpr int WQ_THREADS = 256;
 constexpr int WQ_PMAX = 592;             // partial maxima (CTAs of the first launch)
 
+using biloco::qm::max_nan;               // (a NaN reaches the tensor's maximum, which then gives a tensor scale of 1)
+
 __device__ __forceinline__ float warp_max(float m) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
     return m;
 }
 
@@ -35,14 +37,14 @@ __global__ void __launch_bounds__(WQ_THREADS) weight_amax_kernel(const float4* _
 #pragma unroll 8
     for (long long i = (long long)blockIdx.x * WQ_THREADS + threadIdx.x; i < nvec; i += stride) {
         const float4 a = X[i];
-        m = fmaxf(m, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))));
+        m = max_nan(m, max_nan(max_nan(fabsf(a.x), fabsf(a.y)), max_nan(fabsf(a.z), fabsf(a.w))));
     }
     m = warp_max(m);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int i = 1; i < WQ_THREADS / 32; ++i) m = fmaxf(m, red[i]);
+        for (int i = 1; i < WQ_THREADS / 32; ++i) m = max_nan(m, red[i]);
         pmax[blockIdx.x] = m;
     }
 }
@@ -56,13 +58,13 @@ __global__ void __launch_bounds__(WQ_THREADS) weight_quant_kernel(const float* _
     float gs;
     if (npmax > 0) {
         float m = 0.f;
-        for (int i = threadIdx.x; i < npmax; i += WQ_THREADS) m = fmaxf(m, pmax[i]);
+        for (int i = threadIdx.x; i < npmax; i += WQ_THREADS) m = max_nan(m, pmax[i]);
         m = warp_max(m);
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
         __syncthreads();
         m = red[0];
 #pragma unroll
-        for (int i = 1; i < WQ_THREADS / 32; ++i) m = fmaxf(m, red[i]);
+        for (int i = 1; i < WQ_THREADS / 32; ++i) m = max_nan(m, red[i]);
         gs = m > 0.f ? __fdiv_rn(m, 6.0f * target) : 1.0f;
         if (blockIdx.x == 0 && threadIdx.x == 0) gscale[0] = gs;
     } else {
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(WQ_THREADS) weight_quant_kernel(const float* _
                 x[4 * q] = a.x; x[4 * q + 1] = a.y; x[4 * q + 2] = a.z; x[4 * q + 3] = a.w;
             }
             uint2 c;
-            biloco::qm::quant_block16(x, gs, rule, c, s);
+            biloco::qm::quant_block16<true>(x, gs, rule, c, s);
             *reinterpret_cast<uint2*>(codes + (size_t)row * (K >> 1) + b * 8) = c;
         }
         sf[((size_t)(row >> 7) * (kbp >> 2) + (b >> 2)) * 512 + (row & 31) * 16 + ((row >> 5) & 3) * 4 + (b & 3)] = s;

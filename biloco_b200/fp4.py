@@ -109,6 +109,12 @@ def quantize_nvfp4(x: torch.Tensor, rule: str = None, global_scale=None):
     rows, K = x.shape
     if x.is_cuda and rows > 0 and K > 0:
         return _quantize_nvfp4_cuda(x.contiguous(), rule, global_scale)
+    return _quantize_nvfp4_torch(x, rule, global_scale)
+
+
+def _quantize_nvfp4_torch(x, rule, global_scale):
+    """quantize_nvfp4 as tensor operations (x fp32, any device). A NaN makes its block's scale NaN and the tensor scale 1."""
+    rows, K = x.shape
     target = 448.0 if rule == "static_6" else 256.0
     if global_scale is None:
         amax = x.abs().max() if x.numel() else torch.zeros((), device=x.device)

@@ -85,6 +85,27 @@ def test_weight_quantiser_bytes_equal_the_cpu_restatement(rows, K, rule):
         assert torch.equal(got[2].cpu(), want[2])
 
 
+@pytest.mark.parametrize("rule", ["mse", "static_6", "static_4"])
+@pytest.mark.parametrize("special", [(float("nan"),), (float("inf"),), (-float("inf"), float("nan")), ()])
+def test_weight_quantiser_keeps_what_is_not_finite(special, rule):
+    """NaN and infinities, and given tensor scales that are not positive: the bytes of the torch operations on the same device (a
+    NaN's block decodes to NaN, it is not lost in a maximum)."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(130, 80, device="cuda", generator=g) * 0.02
+    x[3, :16] = 0.0
+    for i, v in enumerate(special):
+        x[7 + 60 * i, 37] = v                # one element of a block
+        x[9, 0] = v                          # (both in one block)
+    for gscale in (None, 3e-4, 0.0, -3e-4, float("nan")):
+        want = fp4._quantize_nvfp4_torch(x, rule, gscale)
+        got = fp4.quantize_nvfp4(x, rule, gscale)
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8)), gscale
+    if special and special[-1] != special[-1]:
+        q = fp4.fake_quantize_fp4(x, rule)
+        assert bool(q[7 + 60 * (len(special) - 1), 32:48].isnan().all())
+
+
 @pytest.mark.parametrize("M,K,smooth,norm,swiglu", [
     (1, 64, False, False, False), (1, 28672, False, True, False), (3, 576, True, True, False), (7, 2560, False, False, True),
     (17, 8192, True, False, False),          # sixteen CTAs, two rows per group
