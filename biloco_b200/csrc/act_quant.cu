@@ -8,7 +8,7 @@
 //     t    = bmax / gs                      per 16-element block
 //     sfD  = e4m3_rn_sat(t / D)             D = 6 or 4
 //     d    = f32(sfD) * gs
-//     code = e2m1_rn(xs / d)                round-to-nearest-even on {0,.5,1,1.5,2,3,4,6}, saturating; 0 if d == 0
+//     code = e2m1_rn(xs / d)                round-to-nearest-even on {0,.5,1,1.5,2,3,4,6}, saturating; 0 if d == 0, sign only if xs is NaN
 //     mse rule: err_D = sum_{j=0..15} (xs_j - value(code_j) * d)^2 in index order (separate mul and add);
 //               the block takes D = 4 iff err_4 < err_6.
 // One launch of ONE cluster (up to sixteen CTAs of 256 or 512 threads): a decode batch is at most a few hundred KB and the
@@ -69,9 +69,8 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {      // (exact: bf
 
 // Half a block per lane (lanes 2i and 2i + 1 hold one block): this lane's eight codes and, in both lanes, the block's scale.
 __device__ __forceinline__ uint32_t quant_half(const float (&x)[8], int lane, float gs, int rule, uint8_t& sf) {
-    float bmax = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) bmax = fmaxf(bmax, fabsf(x[j]));
+    uint32_t keep, sign;
+    float bmax = biloco::qm::half_max(x, keep, sign);
     bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
     const float t = __fdiv_rn(bmax, gs);
     uint32_t c[2] = {0u, 0u};
@@ -83,7 +82,7 @@ __device__ __forceinline__ uint32_t quant_half(const float (&x)[8], int lane, fl
         if (cand == 1 && rule == BILOCO_RULE_STATIC_6) continue;
         s[cand] = float_to_e4m3_sat(__fdiv_rn(t, cand == 0 ? 6.0f : 4.0f));
         const float d = __fmul_rn(e4m3_to_float(s[cand]), gs);
-        c[cand] = biloco::qm::codes8(x, d);
+        c[cand] = biloco::qm::codes8(x, d, keep, sign);
         if (rule == BILOCO_RULE_MSE) {
             float v[8], sq[8];
             biloco::qm::e2m1_unpack8(c[cand], v);

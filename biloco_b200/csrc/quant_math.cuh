@@ -3,7 +3,7 @@
 //     t    = bmax / gs                      per 16-element block
 //     sfD  = e4m3_rn_sat(t / D)             D = 6 or 4
 //     d    = f32(sfD) * gs
-//     code = e2m1_rn(x / d)                 round-to-nearest-even on {0,.5,1,1.5,2,3,4,6}, saturating; 0 if d == 0
+//     code = e2m1_rn(x / d)                 round-to-nearest-even on {0,.5,1,1.5,2,3,4,6}, saturating; 0 if d == 0, sign only if x is NaN
 //     mse rule: err_D = sum_{j=0..15} (x_j - value(code_j) * d)^2 in index order (separate multiply and add);
 //               the block takes D = 4 iff err_4 < err_6.
 #pragma once
@@ -105,10 +105,36 @@ __device__ __forceinline__ void e2m1_unpack8(uint32_t w, float* v) {
     }
 }
 
+// The larger of two values; NaN if either is (fmaxf drops it).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+
+// Largest |x_j| of half a block (NaN elements left out) and, for its codes, what a NaN element's code is: its sign bit over zero. The
+// conversion instructions would make it 6. `keep` has the other elements' nibbles, `sign` the NaN elements' sign bits.
+__device__ __forceinline__ float half_max(const float* x, uint32_t& keep, uint32_t& sign) {
+    float m = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = max_nan(m, fabsf(x[j]));
+    keep = 0xffffffffu;
+    sign = 0u;
+    if (m != m) {
+        m = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            m = fmaxf(m, fabsf(x[j]));
+            if (x[j] != x[j]) { keep &= ~(15u << (4 * j)); sign |= (__float_as_uint(x[j]) >> 31) << (4 * j + 3); }
+        }
+    }
+    return m;
+}
+
 // Codes e2m1_rn(x_j / d) of half a block. The quotients are not formed: x_j times the reciprocal, made 2^-20 smaller and 2^-20
 // larger (more than the few 2^-24 the product can be off by), gives the same code both ways unless the quotient lies at a
 // rounding boundary; only then (about one half block in 12000 on random data) are the IEEE quotients taken.
-__device__ __forceinline__ uint32_t codes8(const float* x, float d) {
+__device__ __forceinline__ uint32_t codes8(const float* x, float d, uint32_t keep, uint32_t sign) {
     if (!(d > 0.f)) return 0u;
     float q[8];
     if (d > 1e-30f && d < 1e30f) {
@@ -118,29 +144,27 @@ __device__ __forceinline__ uint32_t codes8(const float* x, float d) {
         const uint32_t lo = e2m1_pack8(q);
 #pragma unroll
         for (int j = 0; j < 8; ++j) q[j] = x[j] * rh;
-        if (lo == e2m1_pack8(q)) return lo;
+        if (lo == e2m1_pack8(q)) return (lo & keep) | sign;
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) q[j] = __fdiv_rn(x[j], d);
-    return e2m1_pack8(q);
-}
-__device__ __forceinline__ uint2 codes16(const float (&x)[16], float d) { return make_uint2(codes8(x, d), codes8(x + 8, d)); }
-
-// The larger of two values; NaN if either is (fmaxf drops it).
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float m;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
-    return m;
+    return (e2m1_pack8(q) & keep) | sign;
 }
 
 // One thread, one block of sixteen values (the throughput form: thousands of blocks): the arithmetic of the file header.
 // KEEP_NAN (weights): a NaN makes the block's maximum and with it its scale NaN (0x7f, codes 0), and a tensor scale that is not
-// positive gives a scale of zero, as torch's maximum and clamp have it. Otherwise (activations) maxima drop NaN.
+// positive gives a scale of zero, as torch's maximum and clamp have it. Otherwise (activations) the block's maximum and the codes leave NaN elements out.
 template <bool KEEP_NAN>
 __device__ __forceinline__ void quant_block16(const float (&x)[16], float gs, int rule, uint2& codes, uint8_t& sf) {
     float bmax = 0.f;
+    uint32_t keep[2] = {0xffffffffu, 0xffffffffu}, sign[2] = {0u, 0u};
+    if constexpr (KEEP_NAN) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) bmax = KEEP_NAN ? max_nan(bmax, fabsf(x[j])) : fmaxf(bmax, fabsf(x[j]));
+        for (int j = 0; j < 16; ++j) bmax = max_nan(bmax, fabsf(x[j]));
+    } else {
+        bmax = half_max(x, keep[0], sign[0]);
+        bmax = fmaxf(bmax, half_max(x + 8, keep[1], sign[1]));
+    }
     float t = __fdiv_rn(bmax, gs);
     if (KEEP_NAN && t <= 0.f) t = 0.f;
     uint2 c[2];
@@ -152,7 +176,7 @@ __device__ __forceinline__ void quant_block16(const float (&x)[16], float gs, in
         if (cand == 1 && rule == 0) continue;
         s[cand] = float_to_e4m3_sat(__fdiv_rn(t, cand == 0 ? 6.0f : 4.0f));
         const float d = __fmul_rn(e4m3_to_float(s[cand]), gs);
-        c[cand] = codes16(x, d);
+        c[cand] = make_uint2(codes8(x, d, keep[0], sign[0]), codes8(x + 8, d, keep[1], sign[1]));
         if (rule == 2) {
             float v[16];
             e2m1_unpack8(c[cand].x, v);

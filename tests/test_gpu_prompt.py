@@ -133,3 +133,33 @@ def test_activation_quantiser_splits(M, K, smooth, norm, swiglu):
         p, sf, gs = fp4.quantize_nvfp4(q["X"].float().cpu(), "mse")
         assert torch.equal(q["A"][0].cpu(), p) and torch.equal(q["gscale"].cpu(), gs)
         assert torch.equal(q["A_sf"].view(torch.uint8).cpu(), sf.view(torch.uint8))
+
+
+@pytest.mark.parametrize("rule", ["mse", "static_6", "static_4"])
+@pytest.mark.parametrize("M,K", [(1, 64), (5, 512), (32, 2560)])
+def test_activation_quantiser_leaves_nan_elements_out(M, K, rule):
+    """A NaN element gets the code of a zero with its sign and counts for no maximum; a block that holds one keeps the divisor 6 under
+    the mse rule (both errors are NaN, and the comparison takes 4 only where its error is smaller)."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    bits = x.view(torch.int16)
+    spots = [(0, 3, 0x7FC0), (M - 1, K - 1, -0x40), (M // 2, K // 2, 0x7F81), (M // 2, K // 2 + 8, -0x7F)]      # (either sign, both halves of a block)
+    for r, c, v in spots:
+        bits[r, c] = v
+    if K > 64:
+        x[0, 32:48] = float("nan")           # a block of nothing else
+    nan = x.isnan()
+    q = fp4.quantize_activation(x, rule)
+    clean = torch.where(nan, torch.zeros_like(x), x).float()
+    gs = q["gscale"]
+    p, sf, want_gs = fp4.quantize_nvfp4(clean, rule)
+    p6, sf6, _ = fp4.quantize_nvfp4(clean, "static_6", want_gs) if rule == "mse" else (p, sf, None)
+    assert torch.equal(gs, want_gs)
+    blk = nan.view(M, K // 16, 16).any(-1)
+    s = torch.where(blk, fp4.unswizzle_scales(sf6, M, K), fp4.unswizzle_scales(sf, M, K))
+    assert torch.equal(fp4.unswizzle_scales(q["A_sf"], M, K), s)
+    codes = lambda t: torch.stack([t & 15, t >> 4], -1).view(M, K)
+    want = torch.where(blk.repeat_interleave(16, 1), codes(p6), codes(p))
+    live = s.view(torch.float8_e4m3fn).float().repeat_interleave(16, 1) * gs > 0
+    want = torch.where(nan, torch.where((bits < 0) & live, 8, 0).to(torch.uint8), want)
+    assert torch.equal(codes(q["A"][0]), want)
