@@ -96,6 +96,7 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, Ctrl* c
 constexpr int Q_THREADS = 256;
 
 // pmax[CTA] = max |x| over the CTA's share; with smoothing Xs = bf16(x / smooth) is formed here (the maximum is its maximum).
+// A NaN is the maximum and makes the tensor scale 1 (fp4.activation_scale_from_amax).
 __global__ void __launch_bounds__(Q_THREADS) amax_kernel(const uint4* __restrict__ X, const uint4* __restrict__ smooth, uint4* __restrict__ Xs,
                                                          float* __restrict__ pmax, long long nvec, int kvec) {
     __shared__ float red[Q_THREADS / 32];
@@ -114,18 +115,18 @@ __global__ void __launch_bounds__(Q_THREADS) amax_kernel(const uint4* __restrict
         for (int e = 0; e < 4; ++e) {
             float lo, hi;
             qm::unpack_smoothed(w[e], v[e], smooth != nullptr, lo, hi);
-            m = fmaxf(m, fmaxf(fabsf(lo), fabsf(hi)));
+            m = qm::max_nan(m, qm::max_nan(fabsf(lo), fabsf(hi)));
             o[e] = (__float_as_uint(lo) >> 16) | (__float_as_uint(hi) & 0xFFFF0000u);
         }
         if (smooth) Xs[i] = make_uint4(o[0], o[1], o[2], o[3]);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = qm::max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int i = 1; i < Q_THREADS / 32; ++i) m = fmaxf(m, red[i]);
+        for (int i = 1; i < Q_THREADS / 32; ++i) m = qm::max_nan(m, red[i]);
         pmax[blockIdx.x] = m;
     }
 }
@@ -138,14 +139,14 @@ __global__ void __launch_bounds__(Q_THREADS) quant_kernel(const __nv_bfloat16* _
     griddep_launch_dependents();
     griddep_wait();
     float m = 0.f;
-    for (int i = threadIdx.x; i < npmax; i += Q_THREADS) m = fmaxf(m, pmax[i]);
+    for (int i = threadIdx.x; i < npmax; i += Q_THREADS) m = qm::max_nan(m, pmax[i]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = qm::max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     m = red[0];
 #pragma unroll
-    for (int i = 1; i < Q_THREADS / 32; ++i) m = fmaxf(m, red[i]);
+    for (int i = 1; i < Q_THREADS / 32; ++i) m = qm::max_nan(m, red[i]);
     const float gs = m > 0.f ? __fdiv_rn(m, 6.0f * target) : 1.0f;
     if (blockIdx.x == 0 && threadIdx.x == 0) alpha_out[0] = __fmul_rn(w_gscale[0], gs);
     const int kb_row = K >> 4, nkt = K >> 8;

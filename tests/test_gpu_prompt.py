@@ -67,6 +67,29 @@ def test_prompt_matches_exact_value(rows, K, N, R, smooth, bias):
     assert st[0] == 0
 
 
+@pytest.mark.parametrize("R", [0, 32])
+def test_prompt_with_a_nan(R):
+    """One NaN element: the tensor scale is what fp4.activation_scale_from_amax makes of a NaN maximum (1); rows without a NaN have the
+    value of that quantisation, the row with it is NaN where its low-rank term is."""
+    rows, K, N = 70, 512, 136
+    ops = BiLoCoLinear.synthetic(K, N, max(R, 1), "cuda", seed=4).export_operands()
+    if R == 0:
+        ops["V_packed"], ops["U_packed"], ops["S"] = ops["V_packed"][:0], ops["U_packed"][:0], ops["S"][:0]
+    layer = BiLoCoLinear.from_operands(ops)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(rows, K, device="cuda", generator=g).to(torch.bfloat16)
+    x[41, 100] = float("nan")
+    y = layer(x)
+    gs = fp4.activation_scale_from_amax(x.float().abs().max().reshape(1))
+    ok = torch.arange(rows, device="cuda") != 41
+    p, sf, _ = fp4.quantize_nvfp4(x[ok].float(), fp4.CONFIG_X, gs)
+    want = fp4.dequantize_nvfp4(p, sf, gs).double() @ fp4.dequantize_nvfp4(layer.W_codes, layer.W_sf.view(torch.float8_e4m3fn), layer.w_gscale).double().T
+    if R:
+        want = want + ((x[ok].double() @ kernel.unpack_signs(layer.V_packed).double().T) * layer.S.double()) @ kernel.unpack_signs(layer.U_packed).double()
+    assert float(torch.linalg.norm(y[ok].double() - want) / torch.linalg.norm(want)) <= 2e-3       # (bf16 rounding; the derived scale gives 0.1)
+    assert bool(y[41].isnan().all()) == bool(R)
+
+
 @pytest.mark.parametrize("rule", ["mse", "static_6", "static_4"])
 @pytest.mark.parametrize("rows,K", [(1, 16), (127, 48), (129, 336), (300, 1024)])
 def test_weight_quantiser_bytes_equal_the_cpu_restatement(rows, K, rule):
