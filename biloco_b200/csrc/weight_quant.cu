@@ -14,6 +14,7 @@
 #include "quant_math.cuh"
 
 extern "C" int biloco_internal_use_pdl();
+extern "C" void biloco_internal_mark_relayout(cudaStream_t stream);      // (fused_linear.cu: the next fused launch on this stream starts plain)
 
 namespace {
 
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(WQ_THREADS) weight_amax_kernel(const float4* _
 __global__ void __launch_bounds__(WQ_THREADS) weight_quant_kernel(const float* __restrict__ X, const float* __restrict__ pmax, int npmax, float* __restrict__ gscale,
                                                                   uint8_t* __restrict__ codes, uint8_t* __restrict__ sf, int rows, int K, int rule, float target) {
     __shared__ float red[WQ_THREADS / 32];
-    biloco::griddep_launch_dependents();
+    biloco::griddep_launch_dependents();     // (a fused launch, which reads the codes ahead of its wait, goes out plain after this: mark_relayout)
     biloco::griddep_wait();
     float gs;
     if (npmax > 0) {
@@ -124,6 +125,9 @@ extern "C" int biloco_b200_weight_quant(const float* X, void* ws, void* codes, v
     g = (total + WQ_THREADS - 1) / WQ_THREADS;
     if (g > 8ll * sms) g = 8ll * sms;
     cfg.gridDim = dim3((unsigned)g);
-    return cudaLaunchKernelEx(&cfg, weight_quant_kernel, X, (const float*)ws, g1, gscale, (uint8_t*)codes, (uint8_t*)sf, rows, K, rule,
-                              rule == BILOCO_RULE_STATIC_6 ? 448.0f : 256.0f) == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
+    if (cudaLaunchKernelEx(&cfg, weight_quant_kernel, X, (const float*)ws, g1, gscale, (uint8_t*)codes, (uint8_t*)sf, rows, K, rule,
+                           rule == BILOCO_RULE_STATIC_6 ? 448.0f : 256.0f) != cudaSuccess)
+        return BILOCO_ERR_CUDA;
+    biloco_internal_mark_relayout((cudaStream_t)stream);
+    return BILOCO_OK;
 }

@@ -397,10 +397,11 @@ int biloco_b200_read_status(const void* scratch, int32_t* out16, biloco_stream_t
  * The reference launches with a "pdl" flag as well (csrc/biloco_gemm.cu:3421-3429). */
 /* Contract that comes with it: the fused kernels read their STATIC operands (W_codes / W_sf / W_tiled, V_packed, U_col32,
  * S) before that wait, so these must be complete before the kernel that precedes the fused launch on the stream begins.
- * The library's own re-layout calls (biloco_b200_tile_weights, biloco_b200_tile_weights_slab, biloco_b200_pack_u_col32)
- * are covered: the first fused launch that follows one of them on the same stream is issued as a plain launch. A caller
- * that writes these operands with a kernel of its own directly in front of a fused launch sets BILOCO_OPT_PDL to 0 for
- * that launch (or puts any other kernel in between). Activations, alpha, C and the scratch are read after the wait. */
+ * The library's own calls that write such operands (biloco_b200_tile_weights, biloco_b200_tile_weights_slab,
+ * biloco_b200_pack_u_col32, biloco_b200_weight_quant) are covered: the first fused launch that follows one of them on the same
+ * stream, with or without activation quantisers in between, is issued as a plain launch. A caller that writes these
+ * operands with a kernel of its own in front of a fused launch sets BILOCO_OPT_PDL to 0 for that launch; an activation quantiser in
+ * between is enough only if that kernel does not let its successors start early (the quantiser does). Activations, alpha, C and the scratch are read after the wait. */
 #define BILOCO_OPT_PDL 1
 /* Pipeline stages the fused kernel keeps in flight. 0 (default): chosen by the library - for M <= 8 with dependent
  * launch on, a ring of 4 stages so that two consecutive launches are resident on an SM at the same time (the second

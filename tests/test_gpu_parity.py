@@ -436,6 +436,46 @@ def test_fused_directly_after_relayout(kernel, lib, mode):
         check_against_unfused(y[:M].float().cpu().numpy(), y_ref, f"mode {mode}, call {it} directly after the re-layout")
 
 
+@pytest.mark.parametrize("M,between", [(1, False), (1, True), (8, False), (8, True), (32, True)])
+def test_fused_directly_after_weight_quantiser(kernel, lib, M, between):
+    """biloco_b200_weight_quant followed by the fused launch on the row-major codes it writes (W_tiled = NULL), nothing or an activation
+    quantiser in between: the fused launch must not read the codes ahead of the quantiser's end. Bits of the same launch on an
+    idle device."""
+    K, N, R = 5120, 5120, 128
+    g = torch.Generator(device="cuda").manual_seed(M)
+    W = torch.randn(N, K, device="cuda", generator=g) * 0.02
+    p = orc.random_problem(M, K, 128, R, scales="random", seed=7)
+    t = dev_problem(p)
+    U = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, R // 32), device="cuda", dtype=torch.int64, generator=g).to(torch.int32)
+    stream = torch.cuda.current_stream().cuda_stream
+    scratch = torch.zeros(lib.biloco_b200_scratch_bytes(M, N, K, R, 0) // 4, device="cuda")
+    ws = torch.empty(lib.biloco_b200_weight_quant_ws_bytes(), device="cuda", dtype=torch.uint8)
+    gs, ags, alpha = torch.empty(1, device="cuda"), torch.empty(1, device="cuda"), torch.full((1,), 1e-3, device="cuda")
+    A, A_sf = torch.empty(M, K // 2, device="cuda", dtype=torch.uint8), torch.empty(128 * K // 16, device="cuda", dtype=torch.uint8)
+
+    def quantise_activation(flags):
+        return lib.biloco_b200_act_quant(t["X"].data_ptr(), None, None, A.data_ptr(), A_sf.data_ptr(), ags.data_ptr(), None, None, M, M, K, 2 | flags, stream)
+    assert quantise_activation(0) == 0
+
+    def launch(codes, sf, y):
+        return lib.biloco_b200_fused_linear(codes.data_ptr(), sf.data_ptr(), None, alpha.data_ptr(), A.data_ptr(), A_sf.data_ptr(), t["X"].data_ptr(),
+                                            t["V_packed"].data_ptr(), U.data_ptr(), t["S"].data_ptr(), None, y.data_ptr(), scratch.data_ptr(),
+                                            scratch.numel() * 4, M, M, N, K, R, 2, 1, stream)
+    for it in range(4):
+        codes = torch.full((N, K // 2), 0x77, device="cuda", dtype=torch.uint8)        # stale bytes a too-early read would see
+        sf = torch.full((N * K // 16,), 0x48, device="cuda", dtype=torch.uint8)
+        y, again = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16), torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        assert lib.biloco_b200_weight_quant(W.data_ptr(), ws.data_ptr(), codes.data_ptr(), sf.data_ptr(), gs.data_ptr(), N, K, 2, stream) == 0
+        if between:
+            assert quantise_activation(0x200) == 0
+        assert launch(codes, sf, y) == 0
+        torch.cuda.synchronize()
+        assert launch(codes, sf, again) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(y, again) and bool(y.isfinite().all())
+
+
 def test_reference_layout_arguments_are_ignored(kernel):
     """A caller written against the reference passes ITS internal-layout tensors (pack_v_perm bytes as V_perm, a Diag
     buffer, Corr / Cnt scratch) to the mode operators; they are accepted and ignored, and the result is the same as
