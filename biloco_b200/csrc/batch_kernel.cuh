@@ -7,10 +7,10 @@
 //    the dependency wait: static) and multiplies them with its slice of X; partial sums go to global memory, every item's CTA adds a
 //    share of its rank block's outputs over the slices in order and publishes z. On CUDA cores this took most of a launch
 //    from eight rows on, as a launch of its own in front it cost two grid hand-overs.
-//  * Expansion by MMAs: +-1.0 images of the U bits times z as bf16 high part and remainder, the two side by side as ONE operand of
-//    2 x rows (an MMA costs 41 cycles at N = 16 and 50 at N = 64, so the remainder is nearly free).
-//    The two keep 2^-17 of z: unrounded fp32 outputs are 2.5e-6 off the 64-bit value (1.6e-7 with fp32 expansion on CUDA cores),
-//    bf16 outputs 1.66e-3 either way.
+//  * Expansion by MMAs: +-1.0 images of the U bits times z as a sum of bf16 parts, the parts side by side as ONE operand (an MMA
+//    costs 41 cycles at N = 16 and 50 at N = 64, so further parts are nearly free). Up to eight rows three parts, which
+//    are z itself, as the tile kernel's fp32 expansion has it (fp32 outputs 1.5e-7 off the 64-bit value, 2.4e-6 with two parts; 13.6 ->
+//    13.8 us at 8 rows); from nine rows two, which keep 2^-17 of it (2.5e-6). bf16 outputs are 1.66e-3 off either way.
 //  * A tile's contributors all add: contributor s of n takes rows [s M / n, (s + 1) M / n) of every partial sum. With one finisher
 //    per tile the launch was as long as that CTA's n - 1 rounds of dependent loads after everybody else had left.
 //  * Nothing is announced: partial sums and z carry a validity mark in the lowest mantissa bit (parity of the launch count of
@@ -38,17 +38,22 @@ constexpr int IMG = 16384;                       // +-1.0 image: 128 rows x 64 b
 constexpr int NIMG = 4;                          // images in shared memory at a time
 constexpr int TMEM_COLS = 512;
 constexpr int SF_COL = 64;                       // scale factors of stage s: 32 columns at 64 + 32 s (after two accumulators of 32)
-constexpr int LR_COL = 320;                      // expansion accumulators, 64 columns per segment parity; the first also z's
+constexpr int LR_COL = 320;                      // expansion accumulators, 64 columns per segment parity (LR_N of them used); the first also z's
 static_assert(SF_COL + 32 * MAX_RING <= LR_COL && LR_COL + 128 <= TMEM_COLS, "TMEM columns");
 
 template <int MMA_N> struct Cfg {
     static constexpr int A_TILE = MMA_N * 128;
     static constexpr int STAGE = W_TILE_BYTES + SF_TILE_BYTES + A_TILE + SF_TILE_BYTES;
-    static constexpr int ZB = 2 * MMA_N * 128;   // one z operand: high parts, then remainders, of 64 ranks (z stage: X chunk in the first half)
+    static constexpr int PARTS = MMA_N == 8 ? 3 : 2;                       // bf16 parts of z
+    static constexpr int LR_N = MMA_N == 8 ? 32 : PARTS * MMA_N;           // N of the expansion's MMAs: a multiple of 16 (8 rows: columns 24 .. 31 are not read)
+    // One z operand: 64 ranks of every part, [part][row] (z stage: the X chunk in the first rows). At 8 rows the MMA's last eight rows are
+    // whatever follows (the next operand, the control block): their columns are not read, and 1 KB each would cost a ring stage.
+    static constexpr int ZB = PARTS * MMA_N * 128;
     static constexpr int FIXED = 1024 + NIMG * (IMG + ZB) + 1024;
     static constexpr int RING = (SMEM_BUDGET - FIXED) / STAGE < MAX_RING ? (SMEM_BUDGET - FIXED) / STAGE : MAX_RING;
     static constexpr int SMEM = FIXED + RING * STAGE;
     static_assert(STAGE % 1024 == 0 && RING >= 4, "ring");
+    static_assert(LR_N * 128 <= ZB + 1024 && ZB % 1024 == 0 && LR_N <= 64, "z operands");
 };
 
 struct Params {
@@ -143,6 +148,23 @@ __device__ __forceinline__ void image_half(uint8_t* img, int r, int h, uint32_t 
     uint8_t* row = img + (r >> 3) * 1024 + (r & 7) * 128;
 #pragma unroll
     for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(row + (((4 * h + i) ^ (r & 7)) << 4)) = signs8(bits >> (8 * i));
+}
+
+// The next bf16 part of two values; what is left of them stays behind (exactly; nothing of an infinity). Three parts are cut off, which
+// cannot overflow and leaves nothing after the third; of two the first is rounded, which saves a bit.
+template <int PARTS>
+__device__ __forceinline__ uint32_t next_part(float& z0, float& z1) {
+    uint32_t w;
+    if constexpr (PARTS == 3) {
+        w = (__float_as_uint(z0) >> 16) | (__float_as_uint(z1) & 0xFFFF0000u);
+    } else {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(z0, z1);
+        w = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    const float f0 = __uint_as_float(w << 16), f1 = __uint_as_float(w & 0xFFFF0000u);
+    z0 = fabsf(f0) == INFINITY ? 0.f : z0 - f0;
+    z1 = fabsf(f1) == INFINITY ? 0.f : z1 - f1;
+    return w;
 }
 
 template <int MMA_N>
@@ -332,7 +354,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
         const int r128 = tid & 127, half = tid >> 7;
         const uint32_t quad = (uint32_t)((warp & 3) * 32) << 16;
         const int kbytes = p.K >> 3, nch = p.K >> 6;
-        constexpr uint32_t id_z = make_idesc_bf16(TILE_N, MMA_N < 16 ? 16 : MMA_N), id_lr = make_idesc_bf16(TILE_N, 2 * MMA_N);
+        constexpr uint32_t id_z = make_idesc_bf16(TILE_N, MMA_N < 16 ? 16 : MMA_N), id_lr = make_idesc_bf16(TILE_N, CF::LR_N);
         // (A wait or poll that gives up sets the abort flag, which makes the later ones return at once; nobody leaves early, so that the
         // barriers below always have their 256 threads.)
         uint32_t dpar = 0u, fpar = 0u;           // parity of lr_done's next completion; bit b: of lr_free[b]'s
@@ -494,7 +516,9 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                     for (int i = 0; i < nr; ++i) {
                         const int b = (ib + i) & (NIMG - 1), w = w0 + 2 * (cb + i) + (pc >> 2), e0 = 32 * (w0 + 2 * (cb + i)) + 8 * pc;
                         if (tid < MMA_N * 8) {
-                            uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
+                            uint32_t part[CF::PARTS][4];
+#pragma unroll
+                            for (int k = 0; k < CF::PARTS; ++k) part[k][0] = part[k][1] = part[k][2] = part[k][3] = 0u;
                             if (m < p.M && w < w1 && e0 < p.Rg) {
                                 const float* src = zb + (size_t)m * p.Rpad + e0;
                                 uint32_t v[8];
@@ -509,21 +533,17 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                                     if (!(bad & 1u)) break;
                                     if (poll.expired(ctrl, p, ST_Z)) break;
                                 }
-                                uint32_t h[4], l[4];
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
-                                    const float z0 = e0 + 2 * q < p.Rg ? unmark(v[2 * q]) : 0.f, z1 = e0 + 2 * q + 1 < p.Rg ? unmark(v[2 * q + 1]) : 0.f;
-                                    const __nv_bfloat162 hh = __floats2bfloat162_rn(z0, z1);
-                                    const __nv_bfloat162 ll = __floats2bfloat162_rn(z0 - __low2float(hh), z1 - __high2float(hh));
-                                    h[q] = *reinterpret_cast<const uint32_t*>(&hh);
-                                    l[q] = *reinterpret_cast<const uint32_t*>(&ll);
+                                    float z0 = e0 + 2 * q < p.Rg ? unmark(v[2 * q]) : 0.f, z1 = e0 + 2 * q + 1 < p.Rg ? unmark(v[2 * q + 1]) : 0.f;
+#pragma unroll
+                                    for (int k = 0; k < CF::PARTS; ++k) part[k][q] = next_part<CF::PARTS>(z0, z1);
                                 }
-                                hi = make_uint4(h[0], h[1], h[2], h[3]);
-                                lo = make_uint4(l[0], l[1], l[2], l[3]);
                             }
                             uint8_t* o = zop + b * CF::ZB + (m >> 3) * 1024 + (m & 7) * 128 + ((pc ^ (m & 7)) << 4);
-                            *reinterpret_cast<uint4*>(o) = hi;
-                            *reinterpret_cast<uint4*>(o + MMA_N * 128) = lo;
+#pragma unroll
+                            for (int k = 0; k < CF::PARTS; ++k)
+                                *reinterpret_cast<uint4*>(o + k * MMA_N * 128) = make_uint4(part[k][0], part[k][1], part[k][2], part[k][3]);
                         }
                     }
                     fence_proxy_async();
@@ -556,11 +576,16 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
 #pragma unroll
             for (int i = 0; i < RH; ++i) v[i] *= alpha;
             if (lr) {
-                float a[RH], b[RH];
-                ld_rows<MMA_N>(d2 + quad, half, a);
-                ld_rows<MMA_N>(d2 + quad + MMA_N, half, b);
+                float a[RH], b[RH];              // the smaller parts first
+                ld_rows<MMA_N>(d2 + quad + (CF::PARTS - 1) * MMA_N, half, a);
 #pragma unroll
-                for (int i = 0; i < RH; ++i) v[i] += a[i] + b[i];
+                for (int k = CF::PARTS - 2; k >= 0; --k) {
+                    ld_rows<MMA_N>(d2 + quad + k * MMA_N, half, b);
+#pragma unroll
+                    for (int i = 0; i < RH; ++i) a[i] += b[i];
+                }
+#pragma unroll
+                for (int i = 0; i < RH; ++i) v[i] += a[i];
             }
             tc_fence_before_sync();
             warp_arrive(smem_u32(&ctrl->acc_empty[buf]), lane);

@@ -554,6 +554,38 @@ def test_tuned_mode_measures_and_caches(kernel):
     assert m2 in ok and m2 != 7
 
 
+@pytest.mark.parametrize("M,K,N,R", [(5, 5120, 2560, 512), (7, 2560, 1024, 200), (8, 9728, 384, 1030), (9, 512, 136, 72), (15, 9728, 2560, 128),
+                                     (16, 8192, 1024, 1024), (17, 5120, 2560, 512), (31, 2560, 640, 65), (32, 8192, 1024, 1024)])
+def test_batch_fp32_outputs_against_64_bits(kernel, M, K, N, R):
+    """Unrounded outputs of five to 32 rows against the float64 value of the same operands: edges of the 8 / 16 / 32-row forms, ranks
+    that do not fill a 64-rank chunk, K slices of one and of several rounds, tiles shared by several CTAs. Up to eight rows
+    everything is held in fp32: the bound is four roundings of 2^-24 (measured: 1.4e-7 to 1.7e-7). From nine rows z is two bf16
+    parts, 2^-17 of every z at most, half of that on average (2.5e-6)."""
+    from biloco_b200 import fp4
+    from biloco_b200.layer import BiLoCoLinear
+    ops = BiLoCoLinear.synthetic(K, N, R, "cuda", seed=M).export_operands()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    S = (torch.randn(R, device="cuda", generator=g) * 0.2).to(torch.bfloat16)      # (a low-rank term as large as the FP4 sums)
+    x = torch.randn(M, K, device="cuda", generator=g)
+    x[:, torch.randperm(K, device="cuda", generator=g)[: K // 100]] *= 20
+    x = x.to(torch.bfloat16)
+    q = fp4.quantize_activation(x, "mse", w_gscale=torch.full((1,), 1e-3, device="cuda"), rows=M)
+    one = torch.ones(1, device="cuda")
+    a = fp4.dequantize_nvfp4(q["A"][0][:M], q["A_sf"], one).double()
+    w = fp4.dequantize_nvfp4(ops["W_codes"], ops["W_sf"], one).double()
+    z = (x.double() @ kernel.unpack_signs(ops["V_packed"]).double().T) * S.double()
+    want = (a @ w.T) * q["alpha"].double() + z @ kernel.unpack_signs(ops["U_packed"]).double()
+    gemm = kernel.BiLoCoGemm(ops["W_codes"], ops["W_sf"], q["alpha"], ops["V_packed"], ops["U_packed"], S, M=M, mode=2)
+    gemm.fp32_out = True
+    first = None
+    for _ in range(3):                       # (the marks of the exchanged values alternate from launch to launch)
+        y = gemm(q["A"], q["A_sf"], q["X"], A_rec=q.get("A_rec")).view(-1, N)[:M].clone()
+        first = y if first is None else first
+        assert torch.equal(y, first) and gemm.status()[0] == 0
+    rel = float((y.double() - want).norm() / want.norm())
+    assert rel <= (2.4e-7 if M <= 8 else 4e-6), rel
+
+
 @pytest.mark.parametrize("M,K,N,R,mode", [(32, 5120, 5120, 512, 2), (16, 5120, 5120, 512, 2), (32, 1024, 1024, 128, 2), (32, 2560, 1024, 200, 2),
                                           (24, 256, 640, 72, 2), (32, 5120, 2560, 1024, 2), (8, 5120, 5120, 512, 5), (4, 2048, 1024, 64, 2),
                                           (17, 8192, 1024, 512, 2)])
