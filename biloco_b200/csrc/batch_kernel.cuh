@@ -11,15 +11,17 @@
 //    costs 41 cycles at N = 16 and 50 at N = 64, so further parts are nearly free). Up to eight rows three parts, which
 //    are z itself, as the tile kernel's fp32 expansion has it (fp32 outputs 1.5e-7 off the 64-bit value, 2.4e-6 with two parts; 13.6 ->
 //    13.8 us at 8 rows); from nine rows two, which keep 2^-17 of it (2.5e-6). bf16 outputs are 1.66e-3 off either way.
-//  * A tile's contributors all add: contributor s of n takes rows [s M / n, (s + 1) M / n) of every partial sum. With one finisher
+//  * A tile's contributors all add: contributor s of n takes words [s w / n, (s + 1) w / n) of the w that a partial sum has. With one finisher
 //    per tile the launch was as long as that CTA's n - 1 rounds of dependent loads after everybody else had left.
-//  * Nothing is announced: partial sums and z carry a validity mark in the lowest mantissa bit (parity of the launch count of
-//    this scratch) and are polled themselves, one memory round trip per hand-over. The count is kept as eight words to
-//    which every leaving CTA adds its share of 2^20 (no atomic with a result on the way out).
+//  * Nothing is announced, every hand-over is one memory round trip. Partial sums travel as 16-byte words [three rows' sums | launch count]
+//    that the reader polls itself (one store and one load each, whole or not there); z carries a validity mark in the lowest
+//    mantissa bit (parity of the launch count). The count belongs to this scratch and is kept as eight words to which every
+//    leaving CTA adds its share of 2^20 (no atomic with a result on the way out). Sums are whole fp32 values: with the mark in their
+//    lowest bit too, fp32 outputs of the NVFP4 part alone were 7.8e-8 off (5120 x 5120, 16 rows) instead of 4.9e-8.
 //  * Scale factors are moved to TMEM by two groups of four warps in turn (one group's wait - load - store - arrive chain takes
 //    longer than a unit arrives at HBM speed), and the MMA warp waits on one barrier per unit.
 //
-// Measured (us per call, captured chain of distinct layers, K = N = 5120, r = 512, rows 8 / 16 / 32): 13.5 / 14.6 / 17.4 against
+// Measured (us per call, captured chain of distinct layers, K = N = 5120, r = 512, rows 8 / 16 / 32): 13.8 / 14.5 / 16.4 against
 // 20.4 / 24.4 / 29.9 with z on CUDA cores (8) or as a launch of its own (16, 32) and one finisher per tile.
 #pragma once
 #include "fused_cfg.cuh"
@@ -49,12 +51,16 @@ template <int MMA_N> struct Cfg {
     // One z operand: 64 ranks of every part, [part][row] (z stage: the X chunk in the first rows). At 8 rows the MMA's last eight rows are
     // whatever follows (the next operand, the control block): their columns are not read, and 1 KB each would cost a ring stage.
     static constexpr int ZB = PARTS * MMA_N * 128;
+    // Rows of a column that a thread reads from TMEM (its half's; all eight at 8 rows), and 16-byte words of three rows' sums per column.
+    static constexpr int RH = MMA_N / 2, VR = MMA_N == 8 ? 8 : RH, HW = (RH + 2) / 3, SW = MMA_N == 8 ? 3 : 2 * HW;
     static constexpr int FIXED = 1024 + NIMG * (IMG + ZB) + 1024;
     static constexpr int RING = (SMEM_BUDGET - FIXED) / STAGE < MAX_RING ? (SMEM_BUDGET - FIXED) / STAGE : MAX_RING;
     static constexpr int SMEM = FIXED + RING * STAGE;
     static_assert(STAGE % 1024 == 0 && RING >= 4, "ring");
     static_assert(LR_N * 128 <= ZB + 1024 && ZB % 1024 == 0 && LR_N <= 64, "z operands");
 };
+
+constexpr int sum_words(int mma_n) { return mma_n == 8 ? Cfg<8>::SW : (mma_n == 16 ? Cfg<16>::SW : Cfg<32>::SW); }
 
 struct Params {
     const uint8_t *W_tiled, *W_sf, *A_sf, *A_rec;
@@ -67,8 +73,8 @@ struct Params {
     int32_t* status;
     uint32_t* count;          // eight words: launches completed on this scratch, in bits 20.. of their sum
     float* zbuf;              // [32][Rpad]
-    float* zpart;             // [item][MMA_N][128]
-    float* part;              // [tile][slot][MMA_N][128]
+    uint4* zpart;             // [item][SW][128]
+    uint4* part;              // [tile][slot][SW][128]
     uint2* const* ar_recv;    // row-parallel use, see FusedParams
     const uint32_t* ar_counter;
     int ar_world, ar_rank, ar_slot;
@@ -122,6 +128,17 @@ __device__ __forceinline__ void epi_sync() { named_bar_sync(1, EPI_THREADS); }
 __device__ __forceinline__ float mark(float v, uint32_t phase) { return __uint_as_float((__float_as_uint(v) & ~1u) | phase); }
 __device__ __forceinline__ float unmark(uint32_t w) { return __uint_as_float(w & ~1u); }
 
+// Three rows' sums and the launch count as one 128-bit access.
+__device__ __forceinline__ void st_sums(uint4* dst, float a, float b, float c, uint32_t tag) {
+    const uint64_t lo = ((uint64_t)__float_as_uint(b) << 32) | __float_as_uint(a), hi = ((uint64_t)tag << 32) | __float_as_uint(c);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(dst), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ uint4 ld_sums(const uint4* src) {
+    uint64_t lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}" : "=l"(lo), "=l"(hi) : "l"(src) : "memory");
+    return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+
 // polls a failed attempt's time: true = give up
 struct Poll {
     uint64_t t0 = 0;
@@ -167,21 +184,71 @@ __device__ __forceinline__ uint32_t next_part(float& z0, float& z1) {
     return w;
 }
 
-template <int MMA_N>
-__device__ __forceinline__ void ld_rows(uint32_t taddr, int half, float (&v)[MMA_N / 2]) {      // this half's rows of an accumulator
-    if constexpr (MMA_N == 8) {
-        float t[8];
-        tmem_ld_x8(taddr, t);
-        tc_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = half ? t[4 + i] : t[i];
-    } else if constexpr (MMA_N == 16) {
-        tmem_ld_x8(taddr + 8 * half, v);
-        tc_wait_ld();
-    } else {
-        tmem_ld_x16(taddr + 16 * half, v);
-        tc_wait_ld();
+// Words of three rows' sums of a column. 16 and 32 rows: half h's thread holds rows h RH + 3 t + {0, 1, 2} (below the half's end) in word
+// h HW + t; 8 rows: rows 3 w + {0, 1, 2} in word w, of half w % 2's thread (three words instead of four). Words without a row below M
+// do not exist: `live` of them do, word(i) is the i-th.
+template <int MMA_N> struct SumWords {
+    using CF = Cfg<MMA_N>;
+    int n0, live;
+    __device__ __forceinline__ explicit SumWords(int M) {
+        n0 = ((MMA_N == 8 || M < CF::RH ? M : CF::RH) + 2) / 3;
+        live = n0 + (MMA_N != 8 && M > CF::RH ? (M - CF::RH + 2) / 3 : 0);
     }
+    __device__ __forceinline__ int word(int i) const { return i < n0 ? i : CF::HW + i - n0; }
+    static __device__ __forceinline__ int row(int w) { return MMA_N == 8 || w < CF::HW ? 3 * w : CF::RH + 3 * (w - CF::HW); }      // the word's first row
+    static __device__ __forceinline__ int rows(int w, int M) {                                                                  // and how many it has
+        const int left = MMA_N == 8 ? 3 : CF::RH - 3 * (w < CF::HW ? w : w - CF::HW);
+        return min(min(3, left), M - row(w));
+    }
+    static __device__ __forceinline__ void put(uint4* column, const float (&v)[CF::VR], int half, int M, uint32_t tag) {
+        constexpr int NW = MMA_N == 8 ? CF::SW : CF::HW;
+#pragma unroll
+        for (int t = 0; t < NW; ++t) {
+            const float b = 3 * t + 1 < CF::VR ? v[3 * t + 1 < CF::VR ? 3 * t + 1 : 0] : 0.f, c = 3 * t + 2 < CF::VR ? v[3 * t + 2 < CF::VR ? 3 * t + 2 : 0] : 0.f;
+            if (MMA_N == 8) {
+                if ((t & 1) == half && 3 * t < M) st_sums(column + t * 128, v[3 * t], b, c, tag);
+            } else if (half * CF::RH + 3 * t < M) {
+                st_sums(column + (half * CF::HW + t) * 128, v[3 * t], b, c, tag);
+            }
+        }
+    }
+    // Sums of a word over n sources `step` words apart, from source `first` on in cyclic order, each polled until it carries the launch count.
+    static __device__ __forceinline__ void add(const uint4* src, int n, size_t step, int first, uint32_t tag, float (&o)[3], Ctrl* c, const Params& p, int code) {
+        o[0] = o[1] = o[2] = 0.f;
+#pragma unroll 1
+        for (int s0 = 0; s0 < n; s0 += 8) {
+            uint4 x[8];
+            Poll poll;
+#pragma unroll 1
+            while (true) {
+                uint32_t bad = 0u;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    x[j] = make_uint4(0u, 0u, 0u, tag);
+                    const int k = s0 + j + first;
+                    if (s0 + j < n) x[j] = ld_sums(src + (size_t)(k < n ? k : k - n) * step);
+                    bad |= x[j].w ^ tag;
+                }
+                if (!bad) break;
+                if (poll.expired(c, p, code)) break;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (s0 + j < n) {
+                    o[0] = __fadd_rn(o[0], __uint_as_float(x[j].x));
+                    o[1] = __fadd_rn(o[1], __uint_as_float(x[j].y));
+                    o[2] = __fadd_rn(o[2], __uint_as_float(x[j].z));
+                }
+        }
+    }
+};
+
+template <int MMA_N>
+__device__ __forceinline__ void ld_rows(uint32_t taddr, int half, float (&v)[Cfg<MMA_N>::VR]) {      // this thread's rows of an accumulator
+    if constexpr (MMA_N == 8) tmem_ld_x8(taddr, v);
+    else if constexpr (MMA_N == 16) tmem_ld_x8(taddr + 8 * half, v);
+    else tmem_ld_x16(taddr + 16 * half, v);
+    tc_wait_ld();
 }
 
 // One output element: residual, rounding, store, and the peers' copies.
@@ -385,7 +452,8 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
             ctrl->seq = (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) >> 20;
             if (PUSH) ctrl->ar_seq = (ld_volatile_u32(p.ar_counter) >> 20) + 1u;
         }
-        uint32_t phase = 0u;
+        const SumWords<MMA_N> words(p.M);
+        uint32_t tag = 0u, phase = 0u;          // this launch's number on this scratch (twelve bits, never zero for the first), its parity
         // ---- z: partial sums of this CTA's items ----
 #pragma unroll 1
         for (int item = cta; p.R > 0 && item < p.nitems; item += gridDim.x) {
@@ -426,50 +494,32 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                 warp_wait(smem_u32(&ctrl->lr_done), dpar, ctrl, p, ST_Z, 1);
                 dpar ^= 1u;
             }
-            phase = (ctrl->seq & 1u) ^ 1u;       // (written before the first round's barrier)
+            tag = ctrl->seq + 1u;                // (written before the first round's barrier)
+            phase = tag & 1u;
             tc_fence_after_sync();
-            float d[RH];
+            float d[CF::VR];
             ld_rows<MMA_N>(tmem + quad + LR_COL, half, d);
             tc_fence_before_sync();
-            float* dst = p.zpart + (size_t)item * MMA_N * 128 + r128;
-#pragma unroll
-            for (int i = 0; i < RH; ++i)
-                if (half * RH + i < p.M) dst[(half * RH + i) * 128] = mark(d[i], phase);
+            SumWords<MMA_N>::put(p.zpart + (size_t)item * CF::SW * 128 + r128, d, half, p.M, tag);
             epi_sync();                          // (the accumulator has been read; the next item may start)
         }
-        if (p.R == 0 || cta >= p.nitems) { epi_sync(); phase = (ctrl->seq & 1u) ^ 1u; }
+        if (p.R == 0 || cta >= p.nitems) { epi_sync(); tag = ctrl->seq + 1u; phase = tag & 1u; }
         // ---- z: this CTA's share of the outputs of its items' rank blocks, over the slices in order ----
 #pragma unroll 1
         for (int item = cta; p.R > 0 && item < p.nitems; item += gridDim.x) {
             const int rb = item / p.nks, ks = item - rb * p.nks;
-            const int E = p.M * 128, e0 = ks * E / p.nks, e1 = (ks + 1) * E / p.nks;
+            const int E = words.live * 128, e0 = ks * E / p.nks, e1 = (ks + 1) * E / p.nks;
 #pragma unroll 1
             for (int e = e0 + tid; e < e1; e += EPI_THREADS) {
-                const int m = e >> 7, r = e & 127, rank = rb * 128 + r;
+                const int w = words.word(e >> 7), r = e & 127, rank = rb * 128 + r, m = words.row(w), nm = words.rows(w, p.M);
                 const float coef = rank < p.R ? __bfloat162float(p.S[rank]) : 0.f;
-                const float* src = p.zpart + (size_t)rb * p.nks * MMA_N * 128 + e;
-                float t = 0.f;
-#pragma unroll 1
-                for (int j = 0; j < p.nks; j += 8) {
-                    uint32_t x[8];
-                    Poll poll;
-#pragma unroll 1
-                    while (true) {
-                        uint32_t bad = 0u;
+                float t[3];
+                words.add(p.zpart + ((size_t)rb * p.nks * CF::SW + w) * 128 + r, p.nks, CF::SW * 128, 0, tag, t, ctrl, p, ST_Z);
+                if (rank < p.R && !ctrl->abort) {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            x[q] = phase;
-                            if (j + q < p.nks) x[q] = ld_volatile_u32(src + (size_t)(j + q) * MMA_N * 128);
-                            bad |= x[q] ^ phase;
-                        }
-                        if (!(bad & 1u)) break;
-                        if (poll.expired(ctrl, p, ST_Z)) break;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (j + q < p.nks) t = __fadd_rn(t, unmark(x[q]));
+                    for (int i = 0; i < 3; ++i)
+                        if (i < nm) p.zbuf[(size_t)(m + i) * p.Rpad + rank] = mark(__fmul_rn(t[i], coef), phase);
                 }
-                if (rank < p.R && !ctrl->abort) p.zbuf[(size_t)m * p.Rpad + rank] = mark(__fmul_rn(t, coef), phase);
             }
         }
 
@@ -571,21 +621,21 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
             }
             epi_sync();
             tc_fence_after_sync();
-            float v[RH];
+            float v[CF::VR];
             ld_rows<MMA_N>(tmem + quad + 32 * buf, half, v);
 #pragma unroll
-            for (int i = 0; i < RH; ++i) v[i] *= alpha;
+            for (int i = 0; i < CF::VR; ++i) v[i] *= alpha;
             if (lr) {
-                float a[RH], b[RH];              // the smaller parts first
+                float a[CF::VR], b[CF::VR];      // the smaller parts first
                 ld_rows<MMA_N>(d2 + quad + (CF::PARTS - 1) * MMA_N, half, a);
 #pragma unroll
                 for (int k = CF::PARTS - 2; k >= 0; --k) {
                     ld_rows<MMA_N>(d2 + quad + k * MMA_N, half, b);
 #pragma unroll
-                    for (int i = 0; i < RH; ++i) a[i] += b[i];
+                    for (int i = 0; i < CF::VR; ++i) a[i] += b[i];
                 }
 #pragma unroll
-                for (int i = 0; i < RH; ++i) v[i] += a[i];
+                for (int i = 0; i < CF::VR; ++i) v[i] += a[i];
             }
             tc_fence_before_sync();
             warp_arrive(smem_u32(&ctrl->acc_empty[buf]), lane);
@@ -593,47 +643,30 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                 if (n < p.N && !ctrl->abort) {
 #pragma unroll
                     for (int i = 0; i < RH; ++i)
-                        if (half * RH + i < p.M) put<PUSH>(p, ctrl, half * RH + i, n, v[i]);
+                        if (half * RH + i < p.M) put<PUSH>(p, ctrl, half * RH + i, n, MMA_N == 8 && half ? v[CF::VR - RH + i] : v[i]);
                 }
             } else {
-                float* dst = p.part + ((size_t)t * p.slots + slot) * MMA_N * 128 + r128;
-#pragma unroll
-                for (int i = 0; i < RH; ++i)
-                    if (half * RH + i < p.M) dst[(half * RH + i) * 128] = mark(v[i], phase);
+                SumWords<MMA_N>::put(p.part + ((size_t)t * p.slots + slot) * CF::SW * 128 + r128, v, half, p.M, tag);
                 if (np == 0) { ptile[0] = t; pslot[0] = slot; pnc[0] = nc; } else { ptile[1] = t; pslot[1] = slot; pnc[1] = nc; }
                 ++np;
             }
         }
-        // ---- this CTA's rows of the tiles it shares ----
+        // ---- this CTA's words of the tiles it shares ----
 #pragma unroll 1
         for (int q = 0; q < np; ++q) {
             const int t = q == 0 ? ptile[0] : ptile[1], slot = q == 0 ? pslot[0] : pslot[1], nc = q == 0 ? pnc[0] : pnc[1];
             const int n = t * TILE_N + r128;
-            const float* src = p.part + (size_t)t * p.slots * MMA_N * 128 + r128;
+            const uint4* src = p.part + (size_t)t * p.slots * CF::SW * 128 + r128;
 #pragma unroll 1
-            for (int m = slot * p.M / nc + half; m < (slot + 1) * p.M / nc; m += 2) {
-                float o = 0.f;
-#pragma unroll 1
-                for (int s0 = 0; s0 < nc; s0 += 8) {
-                    uint32_t x[8];
-                    Poll poll;
-#pragma unroll 1
-                    while (true) {
-                        uint32_t bad = 0u;
+            for (int i = slot * words.live / nc + half; i < (slot + 1) * words.live / nc; i += 2) {
+                const int w = words.word(i), m = words.row(w), nm = words.rows(w, p.M);
+                float o[3];
+                words.add(src + w * 128, nc, CF::SW * 128, nc - 1, tag, o, ctrl, p, ST_TILE);      // (the tile's last contributor first, as the tile kernel's finisher adds)
+                if (n < p.N && !ctrl->abort) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            x[j] = phase;
-                            if (s0 + j < nc) x[j] = ld_volatile_u32(src + ((size_t)(s0 + j) * MMA_N + m) * 128);
-                            bad |= x[j] ^ phase;
-                        }
-                        if (!(bad & 1u)) break;
-                        if (poll.expired(ctrl, p, ST_TILE)) break;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (s0 + j < nc) o = __fadd_rn(o, unmark(x[j]));
+                    for (int k = 0; k < 3; ++k)
+                        if (k < nm) put<PUSH>(p, ctrl, m + k, n, o[k]);
                 }
-                if (n < p.N && !ctrl->abort) put<PUSH>(p, ctrl, m, n, o);
             }
         }
     }

@@ -204,10 +204,11 @@ static bool make_layout(int M, int N, int K, int R, int num_sms, ScratchLayout* 
         if (L->nks > (nch + 3) / 4) L->nks = (nch + 3) / 4;    // (four chunks of 64 k per item: one round of images)
         if ((long long)nrb * L->nks > 0x7fffff) return false;
         L->nitems = nrb * L->nks;
-        off += (size_t)L->nitems * L->mma_n * TILE_N * sizeof(float);
+        off += (size_t)L->nitems * batch::sum_words(L->mma_n) * TILE_N * sizeof(uint4);
     }
     L->off_part = off;
-    off += (size_t)L->ntile * (L->max_slots + (batch_rows ? 1 : 0)) * L->mma_n * TILE_N * sizeof(float);
+    off += batch_rows ? (size_t)L->ntile * (L->max_slots + 1) * batch::sum_words(L->mma_n) * TILE_N * sizeof(uint4)
+                      : (size_t)L->ntile * L->max_slots * L->mma_n * TILE_N * sizeof(float);
     if (batch_rows) L->off_head = off;
     L->total = (off + 255) / 256 * 256;
     return true;
@@ -409,8 +410,8 @@ static int launch_batch(const CUtensorMap& tmW, const CUtensorMap& tmA, const Fu
     p.S = f.S; p.C = f.C; p.Y = f.Y; p.status = f.status;
     p.count = (uint32_t*)(sc + L.off_bcnt);
     p.zbuf = f.zbuf + (size_t)32 * L.Rpad;           // (the first half belongs to the schedules whose marks follow the other count)
-    p.zpart = (float*)(sc + L.off_zpart);
-    p.part = (float*)(sc + L.off_part);
+    p.zpart = (uint4*)(sc + L.off_zpart);
+    p.part = (uint4*)(sc + L.off_part);
     p.ar_recv = f.ar_recv; p.ar_counter = f.ar_counter; p.ar_world = f.ar_world; p.ar_rank = f.ar_rank; p.ar_slot = f.ar_slot;
     p.M = f.M; p.N = f.N; p.K = f.K; p.R = f.R; p.Rw = f.Rw; p.Rpad = f.Rpad; p.ngroups = f.ngroups; p.Rg = f.Rg;
     for (int g = 0; g < 3; ++g) p.gtile[g] = f.gtile[g];

@@ -586,6 +586,25 @@ def test_batch_fp32_outputs_against_64_bits(kernel, M, K, N, R):
     assert rel <= (2.4e-7 if M <= 8 else 4e-6), rel
 
 
+@pytest.mark.parametrize("M,K,N", [(5, 5120, 2560), (8, 9728, 384), (9, 5120, 5120), (16, 5120, 5120), (17, 2560, 640), (32, 5120, 5120)])
+def test_batch_partial_sums_are_whole(kernel, M, K, N):
+    """The NVFP4 part alone (R = 0), unrounded, against 64 bits: what is left is a few fp32 roundings of partial sums that several CTAs
+    exchange. Measured 5e-8 to 7e-8 where a tile has two to four contributors, 1.2e-7 with thirteen (9728 x 384); a partial sum that gives its last bit
+    to a mark makes that 7.8e-8 to 9e-8 and 1.33e-7."""
+    from biloco_b200 import fp4, ops
+    from biloco_b200.layer import BiLoCoLinear
+    op = BiLoCoLinear.synthetic(K, N, 1, "cuda", seed=M).export_operands()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    q = fp4.quantize_activation(x, "mse", w_gscale=torch.full((1,), 1.1e-3, device="cuda"), rows=M)
+    one = torch.ones(1, device="cuda")
+    want = (fp4.dequantize_nvfp4(q["A"][0][:M], q["A_sf"], one).double() @ fp4.dequantize_nvfp4(op["W_codes"], op["W_sf"], one).double().T) * q["alpha"].double()
+    z = torch.zeros(kernel.scratch_bytes(M, N, K, 0) // 4, device="cuda")
+    y = ops._fused(q["A"], op["W_codes"], q["A_sf"], op["W_sf"], q["alpha"], None, None, None, None, z, M, 1, 2, fp32_out=True).view(-1, N)[:M]
+    rel = float((y.double() - want).norm() / want.norm())
+    assert rel <= (1.25e-7 if N == 384 else 7.4e-8), rel
+
+
 @pytest.mark.parametrize("M,K,N,R,mode", [(32, 5120, 5120, 512, 2), (16, 5120, 5120, 512, 2), (32, 1024, 1024, 128, 2), (32, 2560, 1024, 200, 2),
                                           (24, 256, 640, 72, 2), (32, 5120, 2560, 1024, 2), (8, 5120, 5120, 512, 5), (4, 2048, 1024, 64, 2),
                                           (17, 8192, 1024, 512, 2)])
