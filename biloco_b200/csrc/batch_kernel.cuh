@@ -83,6 +83,7 @@ struct Params {
     int nks, nitems;          // z: K slices per rank block, items in all
     uint32_t epoch;
     int fp32_out;
+    int skip_publish;         // test aid: this CTA keeps its partial sums of z to itself (-1: none)
     unsigned long long wait_ns;
 };
 
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
             float d[CF::VR];
             ld_rows<MMA_N>(tmem + quad + LR_COL, half, d);
             tc_fence_before_sync();
-            SumWords<MMA_N>::put(p.zpart + (size_t)item * CF::SW * 128 + r128, d, half, p.M, tag);
+            if (cta != p.skip_publish) SumWords<MMA_N>::put(p.zpart + (size_t)item * CF::SW * 128 + r128, d, half, p.M, tag);
             epi_sync();                          // (the accumulator has been read; the next item may start)
         }
         if (p.R == 0 || cta >= p.nitems) { epi_sync(); tag = ctrl->seq + 1u; phase = tag & 1u; }
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                 const float coef = rank < p.R ? __bfloat162float(p.S[rank]) : 0.f;
                 float t[3];
                 words.add(p.zpart + ((size_t)rb * p.nks * CF::SW + w) * 128 + r, p.nks, CF::SW * 128, 0, tag, t, ctrl, p, ST_Z);
-                if (rank < p.R && !ctrl->abort) {
+                if (rank < p.R) {                // (also after a wait that gave up: every mark has to be this launch's, or the next launch could take an older z for its own)
 #pragma unroll
                     for (int i = 0; i < 3; ++i)
                         if (i < nm) p.zbuf[(size_t)(m + i) * p.Rpad + rank] = mark(__fmul_rn(t[i], coef), phase);

@@ -138,11 +138,11 @@ static unsigned long long* g_stamps = nullptr;   // debug time-stamp buffer for 
 static size_t g_stamps_bytes = 0;
 static size_t g_stamps_seq = 0;
 static int g_trigger = -1;                        // < 0: chosen per launch (see launch())
-static unsigned long long g_wait_ns = WAIT_BUDGET_NS;   // budget of a device-side wait (row-slab schedule)
+static unsigned long long g_wait_ns = WAIT_BUDGET_NS;   // budget of a device-side wait (row-slab schedule, batch and prompt kernels)
 static int g_inflight = 0;                        // row-slab schedule: weight records in flight while the ring fills (0: all)
 static bool slab_coresident() { return g_use_pdl != 0; }      // (two launches side by side on an SM: half of its shared memory each)
 static int g_dbg = 0;                             // row-slab schedule: timing experiments (see SlabParams::dbg)
-static int g_skip_publish = -1;                   // test aid: this CTA of a row-slab launch keeps its z values to itself
+static int g_skip_publish = -1;                   // test aid: this CTA of a row-slab or batch launch keeps its z values to itself
 
 // Streams on which an operand re-layout (tile_weights, tile_weights_slab, pack_u_col32) was the last thing this library
 // enqueued. The fused kernels read their static operands BEFORE griddepcontrol.wait when they are launched with
@@ -419,6 +419,7 @@ static int launch_batch(const CUtensorMap& tmW, const CUtensorMap& tmA, const Fu
     p.nks = L.nks > 0 ? L.nks : 1; p.nitems = L.nitems;
     p.epoch = f.epoch;
     p.fp32_out = (f.mode & 0x400) ? 1 : 0;
+    p.skip_publish = g_skip_publish;
     p.wait_ns = g_wait_ns;
     int grid = L.G > L.nitems ? L.G : L.nitems;
     if (grid > sms) grid = sms;

@@ -416,10 +416,11 @@ int biloco_b200_read_status(const void* scratch, int32_t* out16, biloco_stream_t
  * sign image x z split into two bf16 parts, fp32 accumulation), below on the CUDA cores. */
 #define BILOCO_OPT_LR_TC 4
 /* Budget of a device-side wait in microseconds (default 200 000; <= 0 restores the default). A wait that runs out
- * records its code in the status words and the launch returns (row-slab schedule; the other schedules keep 200 ms).
+ * records its code in the status words and the launch returns (row-slab schedule, schedules 2 and 4 from five rows, prompt forward; the other launches keep 200 ms).
  * Counterpart in the reference: the bounded polls that record codes in Diag[4095] (csrc/biloco_gemm.cu:1149-1151). */
 #define BILOCO_OPT_WAIT_BUDGET_US 5
-/* Test aid for the failure path: CTA `value` of a row-slab launch computes its z values but does not publish them, so
+/* Test aid for the failure path: CTA `value` of a row-slab launch, or of a launch of schedules 2 and 4 from five rows,
+ * computes its z values (partial sums of z) but does not publish them, so
  * that every consumer's poll runs out of its budget (-1, the default: off). */
 #define BILOCO_OPT_SKIP_PUBLISH 6
 /* Row-slab schedule: weight records a CTA keeps in flight while it fills its ring ahead of the dependency wait

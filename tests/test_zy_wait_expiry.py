@@ -59,6 +59,48 @@ def test_z_poll_runs_out_and_scratch_recovers(M):
     assert torch.equal(again.view(torch.int16), clean.view(torch.int16))
 
 
+@pytest.mark.parametrize("M", [8, 16, 32])
+def test_batch_z_poll_runs_out_and_later_launches_are_right(M):
+    """The same for five to 32 rows: one CTA keeps its partial sums of z to itself, the CTAs that add them up give up within the
+    budget. The launches that follow on the SAME scratch, without reset(), are right: no value of the failed launch or of the
+    one before it passes for a later one's."""
+    from biloco_b200 import _lib, kernel
+    lib = _lib.load()
+    K, N, R = 1024, 1024, 512
+    ps = [orc.random_problem(M, K, N, R, scales="random", seed=11 + i) for i in range(2)]
+    ts = [dev_problem(p) for p in ps]
+    t = ts[0]
+    g = kernel.BiLoCoGemm(t["W"], t["W_sf"], t["alpha"], t["V_packed"], t["U_packed"], t["S"], M=M, mode=2)
+
+    def run(i=0):                            # (the second activation goes with the first problem's weights)
+        y = g(ts[i]["A_pad"], ts[i]["A_sf"], ts[i]["X"]).view(-1, N)[:M].clone()
+        torch.cuda.synchronize()
+        return y
+
+    clean = [run(0), run(1)]
+    assert g.status()[0] == 0
+    for before in range(2):                  # (either parity of the launch count)
+        run(1)
+        try:
+            lib.biloco_b200_set_option(_lib.OPT_WAIT_BUDGET_US, 2000)
+            lib.biloco_b200_set_option(_lib.OPT_SKIP_PUBLISH, 0)
+            t0 = time.perf_counter()
+            run(0)
+            dt = time.perf_counter() - t0
+        finally:
+            lib.biloco_b200_set_option(_lib.OPT_SKIP_PUBLISH, -1)
+            lib.biloco_b200_set_option(_lib.OPT_WAIT_BUDGET_US, 0)
+        st = g.status()
+        assert st[0] == ST_Z and st[2] > 0 and dt < 1.0, (st[:4], dt)
+        for i in (0, 1, 0):
+            assert torch.equal(run(i).view(torch.int16), clean[i].view(torch.int16)), (before, i)
+        if before == 0:
+            run(1)
+    g.reset()
+    assert g.status()[0] == 0
+    assert torch.equal(run(0).view(torch.int16), clean[0].view(torch.int16)) and g.status()[0] == 0
+
+
 def test_peer_allreduce_wait_runs_out_and_reports(lib):
     """The peer all-reduce polls its own receive buffer for the peers' words with a time budget. Here a 'group' of two
     with nobody behind rank 1 (its buffer is a second local allocation that nothing reads or writes back): the poll runs
