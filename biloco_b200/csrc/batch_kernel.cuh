@@ -15,7 +15,7 @@
 //    per tile the launch was as long as that CTA's n - 1 rounds of dependent loads after everybody else had left.
 //  * Nothing is announced, every hand-over is one memory round trip. Partial sums travel as 16-byte words [three rows' sums | launch count]
 //    that the reader polls itself (one store and one load each, whole or not there); z carries a validity mark in the lowest
-//    mantissa bit (parity of the launch count). The count belongs to this scratch and is kept as eight words to which every
+//    mantissa bit (parity of the launch count). The count belongs to this scratch and is kept as eight 64-bit words to which every
 //    leaving CTA adds its share of 2^20 (no atomic with a result on the way out). Sums are whole fp32 values: with the mark in their
 //    lowest bit too, fp32 outputs of the NVFP4 part alone were 7.8e-8 off (5120 x 5120, 16 rows) instead of 4.9e-8.
 //  * Scale factors are moved to TMEM by two groups of four warps in turn (one group's wait - load - store - arrive chain takes
@@ -60,6 +60,12 @@ template <int MMA_N> struct Cfg {
     static_assert(LR_N * 128 <= ZB + 1024 && ZB % 1024 == 0 && LR_N <= 64, "z operands");
 };
 
+// Place of CTA c's partial sums of a tile that it shares, cf being the tile's first contributor: along the units either the CTA or the
+// tile of such a segment goes up, so CTA + tile names it, and CTA + first contributor does too (the next shared tile starts with
+// the last contributor of this one). G + min(tiles, G) places, where tiles x contributors would be several times as many.
+__host__ __device__ constexpr int part_places(int ntile, int G) { return G + (ntile < G ? ntile : G); }
+__device__ __forceinline__ int part_base(int t, int cf, int ntile, int G) { return ntile < G ? t : cf; }
+
 constexpr int sum_words(int mma_n) { return mma_n == 8 ? Cfg<8>::SW : (mma_n == 16 ? Cfg<16>::SW : Cfg<32>::SW); }
 
 struct Params {
@@ -71,18 +77,19 @@ struct Params {
     const __nv_bfloat16 *S, *C;
     void* Y;
     int32_t* status;
-    uint32_t* count;          // eight words: launches completed on this scratch, in bits 20.. of their sum
+    unsigned long long* count;      // eight words: launches completed on this scratch, in bits 20.. of their sum
     float* zbuf;              // [32][Rpad]
     uint4* zpart;             // [item][SW][128]
-    uint4* part;              // [tile][slot][SW][128]
+    uint4* part;              // [part_base(tile) + CTA][SW][128]
     uint2* const* ar_recv;    // row-parallel use, see FusedParams
     const uint32_t* ar_counter;
     int ar_world, ar_rank, ar_slot;
     int M, N, K, R, Rw, Rpad, ngroups, Rg, gtile[3];
-    int ntile, nkt, G, slots; // G: CTAs with units
+    int ntile, nkt, G;        // G: CTAs with units
     int nks, nitems;          // z: K slices per rank block, items in all
     uint32_t epoch;
     int fp32_out;
+    int z_cleared;            // zbuf was cleared in front of this launch: its mark is 1, not the count's parity
     int skip_publish;         // test aid: this CTA keeps its partial sums of z to itself (-1: none)
     unsigned long long wait_ns;
 };
@@ -449,12 +456,17 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
         }
         griddep_wait();                          // everything below reads what earlier kernels of the stream wrote
         if (tid == 0) {
-            const uint4 a = ld_volatile_v4(p.count), b = ld_volatile_v4(p.count + 4);
-            ctrl->seq = (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) >> 20;
+            unsigned long long n = 0ull;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint4 a = ld_volatile_v4(reinterpret_cast<const uint4*>(p.count) + i);
+                n += (((unsigned long long)a.y << 32) | a.x) + (((unsigned long long)a.w << 32) | a.z);
+            }
+            ctrl->seq = (uint32_t)(n >> 20);
             if (PUSH) ctrl->ar_seq = (ld_volatile_u32(p.ar_counter) >> 20) + 1u;
         }
         const SumWords<MMA_N> words(p.M);
-        uint32_t tag = 0u, phase = 0u;          // this launch's number on this scratch (twelve bits, never zero for the first), its parity
+        uint32_t tag = 0u, phase = 0u;          // this launch's number on this scratch (from one), its parity
         // ---- z: partial sums of this CTA's items ----
 #pragma unroll 1
         for (int item = cta; p.R > 0 && item < p.nitems; item += gridDim.x) {
@@ -496,7 +508,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                 dpar ^= 1u;
             }
             tag = ctrl->seq + 1u;                // (written before the first round's barrier)
-            phase = tag & 1u;
+            phase = p.z_cleared ? 1u : tag & 1u;
             tc_fence_after_sync();
             float d[CF::VR];
             ld_rows<MMA_N>(tmem + quad + LR_COL, half, d);
@@ -504,7 +516,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
             if (cta != p.skip_publish) SumWords<MMA_N>::put(p.zpart + (size_t)item * CF::SW * 128 + r128, d, half, p.M, tag);
             epi_sync();                          // (the accumulator has been read; the next item may start)
         }
-        if (p.R == 0 || cta >= p.nitems) { epi_sync(); tag = ctrl->seq + 1u; phase = tag & 1u; }
+        if (p.R == 0 || cta >= p.nitems) { epi_sync(); tag = ctrl->seq + 1u; phase = p.z_cleared ? 1u : tag & 1u; }
         // ---- z: this CTA's share of the outputs of its items' rank blocks, over the slices in order ----
 #pragma unroll 1
         for (int item = cta; p.R > 0 && item < p.nitems; item += gridDim.x) {
@@ -526,7 +538,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
 
         // ---- segments: expansion, accumulator, output or partial sum ----
         int seg = 0, ib = 0;                     // ib: images used so far (image ib % NIMG is next)
-        int ptile[2], pslot[2], pnc[2], np = 0;  // partial segments of this CTA (its first and last at most)
+        int ptile[2], pslot[2], pnc[2], pcf[2], np = 0;      // partial segments of this CTA (its first and last at most)
         uint32_t used = 0u;                      // bit b: image b has been read by expansion MMAs before
 #pragma unroll 1
         for (SegWalk sw(u0, u1, p.nkt); !sw.done(); sw.next(), ++seg) {
@@ -647,17 +659,17 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                         if (half * RH + i < p.M) put<PUSH>(p, ctrl, half * RH + i, n, MMA_N == 8 && half ? v[CF::VR - RH + i] : v[i]);
                 }
             } else {
-                SumWords<MMA_N>::put(p.part + ((size_t)t * p.slots + slot) * CF::SW * 128 + r128, v, half, p.M, tag);
-                if (np == 0) { ptile[0] = t; pslot[0] = slot; pnc[0] = nc; } else { ptile[1] = t; pslot[1] = slot; pnc[1] = nc; }
+                SumWords<MMA_N>::put(p.part + (size_t)(part_base(t, cf, p.ntile, p.G) + cta) * CF::SW * 128 + r128, v, half, p.M, tag);
+                if (np == 0) { ptile[0] = t; pslot[0] = slot; pnc[0] = nc; pcf[0] = cf; } else { ptile[1] = t; pslot[1] = slot; pnc[1] = nc; pcf[1] = cf; }
                 ++np;
             }
         }
         // ---- this CTA's words of the tiles it shares ----
 #pragma unroll 1
         for (int q = 0; q < np; ++q) {
-            const int t = q == 0 ? ptile[0] : ptile[1], slot = q == 0 ? pslot[0] : pslot[1], nc = q == 0 ? pnc[0] : pnc[1];
+            const int t = q == 0 ? ptile[0] : ptile[1], slot = q == 0 ? pslot[0] : pslot[1], nc = q == 0 ? pnc[0] : pnc[1], cf = q == 0 ? pcf[0] : pcf[1];
             const int n = t * TILE_N + r128;
-            const uint4* src = p.part + (size_t)t * p.slots * CF::SW * 128 + r128;
+            const uint4* src = p.part + (size_t)(part_base(t, cf, p.ntile, p.G) + cf) * CF::SW * 128 + r128;
 #pragma unroll 1
             for (int i = slot * words.live / nc + half; i < (slot + 1) * words.live / nc; i += 2) {
                 const int w = words.word(i), m = words.row(w), nm = words.rows(w, p.M);
@@ -682,7 +694,7 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
     }
     if (tid == 0) {         // this CTA's share of 2^20
         const uint32_t share = (uint32_t)((((unsigned long long)(cta + 1)) << 20) / gridDim.x) - (uint32_t)((((unsigned long long)cta) << 20) / gridDim.x);
-        asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p.count + (cta & 7)), "r"(share) : "memory");
+        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p.count + (cta & 7)), "l"((unsigned long long)share) : "memory");
     }
     if (warp == MMA_WARP) { tc_fence_after_sync(); tmem_dealloc(tmem, TMEM_COLS); }
 }

@@ -170,10 +170,13 @@ static int mma_n_for(int M) { return M <= 8 ? 8 : (M <= 16 ? 16 : 32); }
 
 struct ScratchLayout {
     size_t off_zcnt, off_tilecnt, off_z, off_arec, off_bcnt, off_zpart, off_part, off_head, total;
+    size_t tile_total;        // with one fp32 partial sum per tile and contributor at every row count (the allocation-free entry point's limit)
     int ntile, nkt, G, max_slots, Rw, Rpad, mma_n, nks, nitems;
 };
 
-static bool make_layout(int M, int N, int K, int R, int num_sms, ScratchLayout* L) {
+// batch_base > 0: the batch kernel's count and partial sums start there (the array of the allocation-free entry point, where calls of
+// any shape follow one another: nothing but those words ever lies behind it, and the count runs on).
+static bool make_layout(int M, int N, int K, int R, int num_sms, ScratchLayout* L, size_t batch_base = 0) {
     if (M < 1 || M > 32 || N < 8 || (N % 8) || K < KT || (K % KT) || R < 0 || num_sms < 1) return false;
     L->mma_n = mma_n_for(M);
     L->ntile = (N + TILE_N - 1) / TILE_N;
@@ -192,24 +195,31 @@ static bool make_layout(int M, int N, int K, int R, int num_sms, ScratchLayout* 
     L->off_arec = off; off += (M <= 2 && K % 512 == 0) ? (size_t)M * K : 0;
     off = (off + 255) / 256 * 256;
     L->off_head = off;                                         // everything whose meaning depends on the launch counts lies in front
-    // split-K partial sums; from BATCH_MIN_ROWS rows also the batch kernel's launch count and z partial sums. Its values carry
-    // validity marks, so the whole scratch is head there.
+    const size_t tile_part = (size_t)L->ntile * L->max_slots * L->mma_n * TILE_N * sizeof(float);
+    L->tile_total = off + tile_part;
+    // split-K partial sums; from BATCH_MIN_ROWS rows also the batch kernel's launch count and z partial sums. Its words carry
+    // launch numbers, so the whole scratch is head there.
     const bool batch_rows = M >= BATCH_MIN_ROWS;
-    L->off_bcnt = off; off += batch_rows ? 256 : 0;
     L->nks = L->nitems = 0;
-    L->off_zpart = off;
-    if (batch_rows && R > 0) {
-        const int nrb = (R + 127) / 128, nch = K / 64;
-        L->nks = num_sms / nrb < 1 ? 1 : num_sms / nrb;
-        if (L->nks > (nch + 3) / 4) L->nks = (nch + 3) / 4;    // (four chunks of 64 k per item: one round of images)
-        if ((long long)nrb * L->nks > 0x7fffff) return false;
-        L->nitems = nrb * L->nks;
-        off += (size_t)L->nitems * batch::sum_words(L->mma_n) * TILE_N * sizeof(uint4);
+    if (!batch_rows) {
+        L->off_bcnt = L->off_zpart = L->off_part = off;
+        off += tile_part;
+    } else {
+        if (batch_base > off) off = batch_base;
+        L->off_bcnt = off; off += 256;
+        L->off_zpart = off;
+        if (R > 0) {
+            const int nrb = (R + 127) / 128, nch = K / 64;
+            L->nks = num_sms / nrb < 1 ? 1 : num_sms / nrb;
+            if (L->nks > (nch + 3) / 4) L->nks = (nch + 3) / 4;    // (four chunks of 64 k per item: one round of images)
+            if ((long long)nrb * L->nks > 0x7fffff) return false;
+            L->nitems = nrb * L->nks;
+            off += (size_t)L->nitems * batch::sum_words(L->mma_n) * TILE_N * sizeof(uint4);
+        }
+        L->off_part = off;
+        off += (size_t)batch::part_places(L->ntile, L->G) * batch::sum_words(L->mma_n) * TILE_N * sizeof(uint4);
+        if (batch_base == 0) L->off_head = off;
     }
-    L->off_part = off;
-    off += batch_rows ? (size_t)L->ntile * (L->max_slots + 1) * batch::sum_words(L->mma_n) * TILE_N * sizeof(uint4)
-                      : (size_t)L->ntile * L->max_slots * L->mma_n * TILE_N * sizeof(float);
-    if (batch_rows) L->off_head = off;
     L->total = (off + 255) / 256 * 256;
     return true;
 }
@@ -408,17 +418,18 @@ static int launch_batch(const CUtensorMap& tmW, const CUtensorMap& tmA, const Fu
     batch::Params p;
     p.W_tiled = f.W_tiled; p.W_sf = f.W_sf; p.A_sf = f.A_sf; p.A_rec = f.A_rec; p.alpha = f.alpha; p.X = f.X; p.Vp = f.Vp; p.Ucol = f.Ucol;
     p.S = f.S; p.C = f.C; p.Y = f.Y; p.status = f.status;
-    p.count = (uint32_t*)(sc + L.off_bcnt);
+    p.count = (unsigned long long*)(sc + L.off_bcnt);
     p.zbuf = f.zbuf + (size_t)32 * L.Rpad;           // (the first half belongs to the schedules whose marks follow the other count)
     p.zpart = (uint4*)(sc + L.off_zpart);
     p.part = (uint4*)(sc + L.off_part);
     p.ar_recv = f.ar_recv; p.ar_counter = f.ar_counter; p.ar_world = f.ar_world; p.ar_rank = f.ar_rank; p.ar_slot = f.ar_slot;
     p.M = f.M; p.N = f.N; p.K = f.K; p.R = f.R; p.Rw = f.Rw; p.Rpad = f.Rpad; p.ngroups = f.ngroups; p.Rg = f.Rg;
     for (int g = 0; g < 3; ++g) p.gtile[g] = f.gtile[g];
-    p.ntile = L.ntile; p.nkt = L.nkt; p.G = L.G; p.slots = L.max_slots + 1;
+    p.ntile = L.ntile; p.nkt = L.nkt; p.G = L.G;
     p.nks = L.nks > 0 ? L.nks : 1; p.nitems = L.nitems;
     p.epoch = f.epoch;
     p.fp32_out = (f.mode & 0x400) ? 1 : 0;
+    p.z_cleared = L.off_head < L.off_bcnt ? 1 : 0;      // (the allocation-free entry point clears its head on every call and lets the count run on)
     p.skip_publish = g_skip_publish;
     p.wait_ns = g_wait_ns;
     int grid = L.G > L.nitems ? L.G : L.nitems;
@@ -707,6 +718,10 @@ static int fused_linear_impl(const void* W_codes, const void* W_sf, const void* 
 // file-scope array below: every GPU that loads this library holds BILOCO_NOALLOC_SCRATCH_BYTES for it until exit.
 // In host code the array's name is only a stand-in; the device address comes from cudaGetSymbolAddress.
 // ---------------------------------------------------------------------------------------------------------------
+// The allocation-free entry point's array: what lies in front of the batch kernel's words (and all that schedules 2 and 4 need below
+// five rows) may take NOALLOC_LIMIT; behind it the count, at most 180 items of z (R <= 23000 by the limit) and 2 x 148 places
+// of 24 KB each: 17.1 MB.
+constexpr size_t NOALLOC_LIMIT = 6 * 1024 * 1024;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[BILOCO_NOALLOC_SCRATCH_BYTES];
 static void* g_noalloc_ptr[64] = {nullptr};                 // per device, filled by the first call on that device
 
@@ -853,8 +868,8 @@ extern "C" int biloco_b200_fused_linear_noalloc(const void* W_codes, const void*
     const int sms = device_sm_count();
     if (sms < 1) return BILOCO_ERR_CUDA;
     ScratchLayout L;
-    if (!make_layout(M, N, K, R, sms, &L)) return BILOCO_ERR_SHAPE;
-    if (L.total > (size_t)BILOCO_NOALLOC_SCRATCH_BYTES) return BILOCO_ERR_LIMIT;     // beyond the built-in scratch
+    if (!make_layout(M, N, K, R, sms, &L, NOALLOC_LIMIT)) return BILOCO_ERR_SHAPE;
+    if (L.tile_total > NOALLOC_LIMIT || L.total > (size_t)BILOCO_NOALLOC_SCRATCH_BYTES) return BILOCO_ERR_LIMIT;     // beyond the built-in scratch
     if (((uintptr_t)W_tiled & 15) || ((uintptr_t)W_codes & 15) || ((uintptr_t)A_codes & 15) || ((uintptr_t)W_sf & 15) ||
         ((uintptr_t)A_sf & 15) || ((uintptr_t)X_bf16 & 15) || ((uintptr_t)U_col32 & 3))
         return BILOCO_ERR_ALIGN;
@@ -869,8 +884,9 @@ extern "C" int biloco_b200_fused_linear_noalloc(const void* W_codes, const void*
     uint8_t* sc = (uint8_t*)g_noalloc_ptr[dev];
 
     // The array keeps what the last call left, possibly from another problem shape or from a call whose wait gave up:
-    // status words, launch count, tile counters and the z area all restart from zero on every call (the z values'
-    // validity marks are relative to the launch count).
+    // status words, the tile kernel's launch count, tile counters and the z area all restart from zero on every call (the z values'
+    // validity marks are relative to a launch count). The batch kernel's count, behind NOALLOC_LIMIT, runs on, and with it the
+    // numbers in its partial sums.
     const size_t clear = L.off_head;
     if (cudaMemsetAsync(sc, 0, clear, s) != cudaSuccess) return BILOCO_ERR_CUDA;
 

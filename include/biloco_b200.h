@@ -366,16 +366,18 @@ int biloco_b200_fused_linear(const void* W_codes, const void* W_sf, const void* 
  * the caller's. Same arithmetic and same results as biloco_b200_fused_linear (arguments as there, minus scratch and
  * epoch), with two restrictions: `mode` is BILOCO_MODE_COUNTER or BILOCO_MODE_OWNER (optionally OR-ed with
  * BILOCO_OUT_FP32); BILOCO_MODE_CLUSTER and BILOCO_MODE_SLAB return BILOCO_ERR_MODE here.
- *   - Limit: problems whose biloco_b200_scratch_bytes(M, N, K, R, 0) exceeds BILOCO_NOALLOC_SCRATCH_BYTES are rejected
- *     with BILOCO_ERR_LIMIT (nothing is enqueued). K = N = 5120 needs 0.8 MB (M <= 8) to 2.8 MB (M = 32).
+ *   - Limit: problems whose status words, counters, z area (256 bytes per rank) and fp32 partial outputs, one per 128-column
+ *     tile and contributing CTA (512 bytes x 8, 16 or 32 rows each), exceed 6 MB are rejected with BILOCO_ERR_LIMIT (nothing is
+ *     enqueued). K = N = 5120, r = 512 takes 0.8 MB (M <= 8) to 2.6 MB (M = 32) of them; 32 rows of 8192 -> 28672, r = 1024: 3.8 MB.
+ *     (From five rows the launch keeps its partial sums in the rest of the array, in another form.)
  *   - The first call on a device looks up the array's device address (a set-up step of a few microseconds): make
  *     that first call outside any stream capture.
  *   - All calls on a device share the one array. It keeps what the previous call left; each call clears, on `stream`,
- *     the words that have to start at zero (a cudaMemsetAsync of up to about 0.3 MB in front of the kernel, which also
+ *     the words that have to start at zero (a cudaMemsetAsync of 256 bytes per rank and a little more in front of the kernel, which also
  *     means that this launch does not start early under the previous kernel of the stream). Two calls that overlap on the GPU (different streams without ordering)
  *     race on it: keep calls to this entry point ordered.
  * No counterpart in the reference (its scratch tensors are allocated by BiLoCoGemm through PyTorch). */
-#define BILOCO_NOALLOC_SCRATCH_BYTES (6 * 1024 * 1024)
+#define BILOCO_NOALLOC_SCRATCH_BYTES (18 * 1024 * 1024)
 int biloco_b200_fused_linear_noalloc(const void* W_codes, const void* W_sf, const void* W_tiled, const float* alpha,
                                      const void* A_codes, const void* A_sf, const void* X_bf16,
                                      const void* V_packed, const int32_t* U_col32, const void* S_bf16,
