@@ -10,11 +10,11 @@
 //   quant_kernel     tensor scale, NVFP4 codes and block scales, one thread per 16-element block, written as the records the
 //                    GEMM stages: per 128 rows and 256 k [codes, 128-byte swizzle applied | four scale atoms], 18 KB
 //   z_gemm_kernel    z on the tensor cores (bf16 x +-1 images of the V bits, K split over a cluster and added through
-//                    distributed shared memory in rank order), divided by alpha and written as bf16 high part + remainder
+//                    distributed shared memory in rank order), divided by alpha and written as bf16 high part + remainders
 //   gemm_kernel      NVFP4 GEMM and, into the SAME accumulator, z times +-1 images of the U bits; epilogue alpha * acc + bias
 //
-// The low-rank term shares the accumulator because z is divided by alpha beforehand (fp32; high + low part keep 2^-17): a
-// second accumulator would not fit TMEM beside 256 columns and the scale factors.
+// The low-rank term shares the accumulator because z is divided by alpha beforehand (fp32; high + low part keep 2^-17, a third part,
+// where there is one, all of it): a second accumulator would not fit TMEM beside 256 columns and the scale factors.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -201,9 +201,9 @@ struct ZParams {
     const uint8_t* Vp;
     const __nv_bfloat16* S;
     const float* alpha;
-    uint8_t* zrec;
+    uint8_t *zrec, *z3;             // z3: third parts of the last row tile, or null
     unsigned long long wait_ns;
-    int rows, K, R, ntr, cs;        // ntr: rank tiles
+    int rows, K, R, nrt, ntr, cs;   // ntr: rank tiles
 };
 template <int NR> struct ZCfg {
     static constexpr int STAGE = 2 * (TM + NR) * 128;         // [X of two chunks | sign images of two chunks]
@@ -361,27 +361,35 @@ __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__
     else __syncthreads();
     if (warp < AUX_WARPS && !ctrl->abort) {
         const float alpha = *p.alpha;
-        const float* part = reinterpret_cast<const float*>(sm);
+        const float* part_sums = reinterpret_cast<const float*>(sm);
         const int nlr = (p.R + 63) >> 6;
+        const bool third = p.z3 != nullptr && rt == p.nrt - 1;
 #pragma unroll 1
         for (int j = half; j < W / 4; j += 2) {          // four ranks at a time
-            uint32_t hi[2], lo[2];
+            uint32_t part[3][2];
             const int col = q * W + 4 * j;               // column of the rank tile
             const int rank = rb * NR + col;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 float a = 0.f;
-                for (int src = 0; src < p.cs; ++src) a = __fadd_rn(a, part[(src * W + 4 * j + i) * TM + row]);
+                for (int src = 0; src < p.cs; ++src) a = __fadd_rn(a, part_sums[(src * W + 4 * j + i) * TM + row]);
                 float z = 0.f;
                 if (rank + i < p.R && alpha != 0.f) z = __fdiv_rn(__fmul_rn(a, __bfloat162float(p.S[rank + i])), alpha);
-                const __nv_bfloat16 h = __float2bfloat16_rn(z), l = __float2bfloat16_rn(z - __bfloat162float(h));
-                const uint32_t hb = __bfloat16_as_ushort(h), lb = __bfloat16_as_ushort(l);
-                if (i & 1) { hi[i >> 1] |= hb << 16; lo[i >> 1] |= lb << 16; } else { hi[i >> 1] = hb; lo[i >> 1] = lb; }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {            // (the remainders are exact; an infinity has none)
+                    if (k == 2 && !third) break;
+                    const __nv_bfloat16 h = __float2bfloat16_rn(z);
+                    const uint32_t hb = __bfloat16_as_ushort(h);
+                    z = fabsf(__bfloat162float(h)) == INFINITY ? 0.f : z - __bfloat162float(h);
+                    if (i & 1) part[k][i >> 1] |= hb << 16; else part[k][i >> 1] = hb;
+                }
             }
             if (rank < nlr * 64) {
-                uint8_t* o = p.zrec + ((size_t)rt * nlr + (rank >> 6)) * Z_REC + row * 128 + (((((rank & 63) >> 3)) ^ (row & 7)) << 4) + (rank & 4) * 2;
-                *reinterpret_cast<uint2*>(o) = make_uint2(hi[0], hi[1]);
-                *reinterpret_cast<uint2*>(o + TM * 128) = make_uint2(lo[0], lo[1]);
+                const int at = row * 128 + (((((rank & 63) >> 3)) ^ (row & 7)) << 4) + (rank & 4) * 2;
+                uint8_t* o = p.zrec + ((size_t)rt * nlr + (rank >> 6)) * Z_REC + at;
+                *reinterpret_cast<uint2*>(o) = make_uint2(part[0][0], part[0][1]);
+                *reinterpret_cast<uint2*>(o + TM * 128) = make_uint2(part[1][0], part[1][1]);
+                if (third) *reinterpret_cast<uint2*>(p.z3 + (size_t)(rank >> 6) * (TM * 128) + at) = make_uint2(part[2][0], part[2][1]);
             }
         }
     }
@@ -401,7 +409,7 @@ __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__
 // ------------------------------------------------------------------------------------------------------------
 struct GParams {
     const uint8_t* arec;
-    const uint8_t* zrec;
+    const uint8_t *zrec, *z3;       // (z3: third parts of z, last row tile only, or null)
     const uint8_t* W_sf;
     const int32_t* Ucol;
     const float* alpha;
@@ -417,7 +425,8 @@ template <int NT> struct GCfg {
     static constexpr int SFB_OFF = KS * A_REC;                                 // [k-tile][block] 2 KB
     static constexpr int B_OFF = SFB_OFF + KS * SFB_BLOCKS * 2048;             // [k-tile] NT x 128 bytes
     static constexpr int FP4_BYTES = B_OFF + KS * NT * 128;
-    static constexpr int LR_BYTES = Z_REC + NT * 128;
+    static constexpr int LR_BYTES = Z_REC + NT * 128;                          // z's two parts, sign image
+    static constexpr bool Z3_FITS = LR_BYTES + TM * 128 <= FP4_BYTES;          // (a third part behind them)
     static constexpr int STAGE = FP4_BYTES > LR_BYTES ? FP4_BYTES : LR_BYTES;
     static constexpr int ST = 3;
     static constexpr int SMEM = 1024 + ST * STAGE + CTRL_BYTES;
@@ -429,7 +438,8 @@ template <int NT> struct GCfg {
     static_assert(SMEM <= 227 * 1024, "shared memory");
 };
 
-template <int NT>
+// THIRD: the last row tile has third parts of z.
+template <int NT, bool THIRD>
 __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ GParams p) {
     using C = GCfg<NT>;
     extern __shared__ uint8_t smem_raw[];
@@ -437,7 +447,12 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
     uint8_t* sm = smem_raw + (base - raw);
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(sm + C::ST * C::STAGE);
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int nkt = p.K >> 8, nfs = (nkt + C::KS - 1) / C::KS, nst = nfs + p.nlr, ntiles = p.nrt * p.nnt;      // nfs: NVFP4 stages
+    const int nkt = p.K >> 8, nfs = (nkt + C::KS - 1) / C::KS, ntiles = p.nrt * p.nnt;      // nfs: NVFP4 stages
+    // Stages of a tile: NVFP4, then 64 ranks each. Where z has a third part (rows of the last row tile) it comes with them, or, where a
+    // stage has no room for it, in stages of its own behind them.
+    auto third_part = [&](int rt) { return THIRD && rt == p.nrt - 1; };
+    auto stages = [&](int rt) { return nfs + p.nlr + (!C::Z3_FITS && third_part(rt) ? p.nlr : 0); };
+    auto rank_stage = [&](int j) { return !THIRD || C::Z3_FITS || j - nfs < p.nlr ? j - nfs : j - nfs - p.nlr; };
     if (tid == 0) {
         for (int s = 0; s < C::ST; ++s) {
             mbar_init(smem_u32(&ctrl->full[s]), 2);      // (both producer warps)
@@ -467,7 +482,7 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
             bool ok = true, first = true;
             for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
                 const int nt = tile / p.nrt, rt = tile - nt * p.nrt;
-                const int n0 = nt * NT, blk0 = n0 >> 7;
+                const int n0 = nt * NT, blk0 = n0 >> 7, nst = stages(rt);
                 const int nblk = NT == 256 && (blk0 + 1) * TM < p.N ? 2 : 1;      // scale blocks that exist
                 const uint8_t* arec = p.arec + (size_t)rt * nkt * A_REC;
                 const uint8_t* zrec = p.zrec + (size_t)rt * p.nlr * Z_REC;
@@ -477,9 +492,12 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
                     const uint32_t st = base + s * C::STAGE, bar = smem_u32(&ctrl->full[s]);
                     const int kt = j * C::KS, nk = nkt - kt < C::KS ? nkt - kt : C::KS;
                     if (warp == PRODUCER_WARP) {
-                        const uint32_t bytes = j < nfs ? nk * A_REC : Z_REC;
-                        mbar_arrive_expect_tx(bar, bytes);
-                        bulk_load(st, j < nfs ? arec + (size_t)kt * A_REC : zrec + (size_t)(j - nfs) * Z_REC, bytes, bar);
+                        const bool alone = THIRD && !C::Z3_FITS && j >= nfs + p.nlr, with = C::Z3_FITS && j >= nfs && third_part(rt);
+                        const uint32_t bytes = j < nfs ? nk * A_REC : (alone ? TM * 128 : Z_REC);
+                        const uint8_t* z3 = p.z3 + (size_t)rank_stage(j) * (TM * 128);
+                        mbar_arrive_expect_tx(bar, bytes + (with ? TM * 128 : 0));
+                        bulk_load(st, j < nfs ? arec + (size_t)kt * A_REC : (alone ? z3 : zrec + (size_t)(j - nfs) * Z_REC), bytes, bar);
+                        if (with) bulk_load(st + C::LR_BYTES, z3, TM * 128, bar);
                     } else if (j < nfs) {
                         mbar_arrive_expect_tx(bar, (uint32_t)(nk * (NT * 128 + nblk * 2048)));
                         tma_load_2d(st + C::B_OFF, &tmW, kt * 128, n0, bar);
@@ -499,6 +517,8 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
         uint32_t par = 0u;
         bool ok = true, ready = false;
         for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, ++ti) {
+            const int rt = tile % p.nrt, nst = stages(rt);
+            const bool third = third_part(rt);
             if (ti > 0 && !warp_wait(smem_u32(&ctrl->acc_empty), (uint32_t)((ti - 1) & 1), ctrl, p.wait_ns, 2, 9)) break;
             for (int j = 0; j < nst; ++j) {
                 if (!ready && !(ok = warp_wait(smem_u32(&ctrl->aux[s]), par, ctrl, p.wait_ns, 2, 10))) break;
@@ -519,11 +539,13 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
                                 tc_mma_nvf4(tmem, ad + 2 * k, bd + 2 * k, id4, sf + 4 * k, sf + 16 + C::SFB_STEP * k, (j > 0 || kk > 0 || k > 0) ? 1u : 0u);
                         }
                     } else {
-                        const uint64_t ad = make_smem_desc(st, 1024, 2), ld = make_smem_desc(st + TM * 128, 1024, 2), bd = make_smem_desc(st + Z_REC, 1024, 2);
+                        const uint64_t ad = make_smem_desc(st, 1024, 2), ld = make_smem_desc(st + TM * 128, 1024, 2), bd = make_smem_desc(st + Z_REC, 1024, 2),
+                                       td = make_smem_desc(st + (C::Z3_FITS ? C::LR_BYTES : 0), 1024, 2);
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             tc_mma_bf16(tmem, ad + 2 * k, bd + 2 * k, id16, 1u);
-                            tc_mma_bf16(tmem, ld + 2 * k, bd + 2 * k, id16, 1u);
+                            if (!THIRD || C::Z3_FITS || j < nfs + p.nlr) tc_mma_bf16(tmem, ld + 2 * k, bd + 2 * k, id16, 1u);
+                            if (THIRD && C::Z3_FITS && third) tc_mma_bf16(tmem, td + 2 * k, bd + 2 * k, id16, 1u);
                         }
                     }
                     tc_commit(smem_u32(&ctrl->empty[s]));
@@ -545,7 +567,7 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
         constexpr int NC = NT >= 128 ? NT / 128 : 1;
         for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, ++ti) {
             const int nt = tile / p.nrt, rt = tile - nt * p.nrt;
-            const int n0 = nt * NT;
+            const int n0 = nt * NT, nst = stages(rt);
             // U words of this thread's columns for its next low-rank stage (64 ranks): requested a stage of its group ahead
             uint32_t u[NC][2];
             auto u_words = [&](int w0, uint32_t (&v)[NC][2]) {
@@ -556,7 +578,7 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
                     for (int h = 0; h < 2; ++h) v[i][h] = (n < p.N && w0 + h < p.Rw) ? (uint32_t)p.Ucol[(size_t)n * p.Rw + w0 + h] : 0u;
                 }
             };
-            u_words(2 * ((it + nfs + g) & 1), u);          // (its first low-rank stage is the tile's first or second)
+            u_words(2 * rank_stage(nfs + ((it + nfs + g) & 1)), u);      // (its first low-rank stage is the tile's first or second)
             for (int j = 0; j < nst; ++j, ++it) {
                 if ((it & 1) == g) {
                     uint8_t* st = sm + s * C::STAGE;
@@ -595,7 +617,7 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
                     } else {
                         // sign image of 64 ranks: row = output column (NT = 64: two threads per column, 32 ranks each)
                         uint32_t un[NC][2];
-                        u_words(2 * (j - nfs + 2), un);
+                        u_words(2 * rank_stage(j + 2), un);
 #pragma unroll
                         for (int i = 0; i < NC; ++i) {
                             const int r = NT == 64 ? t >> 1 : i * 128 + t;
@@ -669,7 +691,7 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
 // ------------------------------------------------------------------------------------------------------------
 // Host side
 // ------------------------------------------------------------------------------------------------------------
-struct Layout { size_t alpha, pmax, xs, arec, zrec, total; int nrt, nlr; };
+struct Layout { size_t alpha, pmax, xs, arec, zrec, z3, total; int nrt, nlr; bool third; };
 constexpr int MAX_PMAX = 592;
 static Layout layout(int rows, int K, int R, bool smooth) {
     Layout L;
@@ -682,6 +704,11 @@ static Layout layout(int rows, int K, int R, bool smooth) {
     L.xs = o; if (smooth) o += up((size_t)rows * K * 2);
     L.arec = o; o += up((size_t)L.nrt * (K / KT) * A_REC);
     L.zrec = o; o += (size_t)L.nrt * L.nlr * Z_REC;
+    // One to eight rows behind the last whole 32 have a third part of z, which is then z itself: taken alone (a decode launch) these rows
+    // have fp32 z too. It costs their row tile half as many low-rank MMAs again (5120 x 5120, r = 512: 33 rows 28.1 -> 30.2 us,
+    // 513 rows 52 -> 57.6, 2049 rows 114 -> 121), and all other row counts nothing.
+    L.third = R > 0 && (rows & 31) >= 1 && (rows & 31) <= 8;
+    L.z3 = o; if (L.third) o += (size_t)L.nlr * TM * 128;
     L.total = o;
     return L;
 }
@@ -725,11 +752,11 @@ static int launch_z(const CUtensorMap& tmX, ZParams z, int nrt, int sms, int dev
     return cudaLaunchKernelEx(&l.cfg, z_gemm_kernel<NR>, tmX, z) == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
 }
 
-template <int NT>
-static int launch_gemm(const void* W, GParams g, int sms, int dev, cudaStream_t s) {
+template <int NT, bool THIRD>
+static int launch_gemm_form(const void* W, GParams g, int sms, int dev, cudaStream_t s) {
     static bool ready[64] = {false};
     if (!ready[dev]) {
-        if (cudaFuncSetAttribute(gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GCfg<NT>::SMEM) != cudaSuccess) return BILOCO_ERR_CUDA;
+        if (cudaFuncSetAttribute(gemm_kernel<NT, THIRD>, cudaFuncAttributeMaxDynamicSharedMemorySize, GCfg<NT>::SMEM) != cudaSuccess) return BILOCO_ERR_CUDA;
         ready[dev] = true;
     }
     CUtensorMap tmW;
@@ -737,15 +764,20 @@ static int launch_gemm(const void* W, GParams g, int sms, int dev, cudaStream_t 
     g.nnt = (g.N + NT - 1) / NT;
     const int tiles = g.nrt * g.nnt;
     Launch l(tiles < sms ? tiles : sms, G_NT, GCfg<NT>::SMEM, s);
-    return cudaLaunchKernelEx(&l.cfg, gemm_kernel<NT>, tmW, g) == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
+    return cudaLaunchKernelEx(&l.cfg, gemm_kernel<NT, THIRD>, tmW, g) == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
+}
+template <int NT>
+static int launch_gemm(const void* W, const GParams& g, int sms, int dev, cudaStream_t s) {
+    return g.z3 ? launch_gemm_form<NT, true>(W, g, sms, dev, s) : launch_gemm_form<NT, false>(W, g, sms, dev, s);
 }
 
 // Estimated cycles of the GEMM with NT columns per tile: waves of (k-stages, each the longer of its MMAs and its loads, low-rank
 // stages, prologue and epilogue). MMA cycles as measured (see elect_one); loads at about 45 bytes per cycle and SM.
-static double gemm_cost(int NT, int mma, int nrt, int N, int nkt, int nlr, int sms) {
+static double gemm_cost(int NT, int mma, int nrt, int N, int nkt, int nlr, int sms, bool third) {
     const int tiles = nrt * ((N + NT - 1) / NT);
     const double load = (A_REC + NT * 128 + (NT >= 128 ? NT / 128 : 1) * 2048) / 45.0, work = 4.0 * mma;
-    return (double)((tiles + sms - 1) / sms) * (nkt * (load > work ? load : work) + nlr * 8.0 * mma + 1500.0 + 6.0 * NT);
+    return (double)((tiles + sms - 1) / sms) * (nkt * (load > work ? load : work) + nlr * 8.0 * mma + 1500.0 + 6.0 * NT)
+           + (third ? nlr * (NT == 256 ? 8.0 * mma : 4.0 * mma) : 0.0);      // (one row tile's third parts; stages of their own at 256 columns)
 }
 
 }  // namespace prompt
@@ -799,15 +831,15 @@ extern "C" int biloco_b200_prompt_linear(const void* W_codes, const void* W_sf, 
     if (R > 0) {
         CUtensorMap tmX;
         if (biloco_internal_encode_map(&tmX, 1, X, rows, K, 64, prompt::TM) != BILOCO_OK) return BILOCO_ERR_CUDA;
-        prompt::ZParams z = {(const uint8_t*)V_packed, (const __nv_bfloat16*)S_bf16, alpha, w + L.zrec, ns, rows, K, R, 0, 0};
+        prompt::ZParams z = {(const uint8_t*)V_packed, (const __nv_bfloat16*)S_bf16, alpha, w + L.zrec, L.third ? w + L.z3 : nullptr, ns, rows, K, R, L.nrt, 0, 0};
         // 128 ranks per tile halve the reads of X; 64 where that would leave the device half empty
         const int rc = (R > 64 && L.nrt * ((R + 127) / 128) * 8 >= sms) ? prompt::launch_z<128>(tmX, z, L.nrt, sms, dev, s) : prompt::launch_z<64>(tmX, z, L.nrt, sms, dev, s);
         if (rc != BILOCO_OK) return rc;
     }
-    prompt::GParams g = {w + L.arec, w + L.zrec, (const uint8_t*)W_sf, U_col32, alpha, (const __nv_bfloat16*)bias_bf16, (__nv_bfloat16*)Y_bf16, ns,
+    prompt::GParams g = {w + L.arec, w + L.zrec, L.third ? w + L.z3 : nullptr, (const uint8_t*)W_sf, U_col32, alpha, (const __nv_bfloat16*)bias_bf16, (__nv_bfloat16*)Y_bf16, ns,
                          rows, N, K, R, (R + 31) / 32, L.nrt, 0, L.nlr};
-    const double c64 = prompt::gemm_cost(64, 50, L.nrt, N, K / 256, L.nlr, sms), c128 = prompt::gemm_cost(128, 66, L.nrt, N, K / 256, L.nlr, sms),
-                 c256 = prompt::gemm_cost(256, 130, L.nrt, N, K / 256, L.nlr, sms);
+    const double c64 = prompt::gemm_cost(64, 50, L.nrt, N, K / 256, L.nlr, sms, L.third), c128 = prompt::gemm_cost(128, 66, L.nrt, N, K / 256, L.nlr, sms, L.third),
+                 c256 = prompt::gemm_cost(256, 130, L.nrt, N, K / 256, L.nlr, sms, L.third);
     if (c256 <= c128 && c256 <= c64) return prompt::launch_gemm<256>(W_codes, g, sms, dev, s);
     if (c128 <= c64) return prompt::launch_gemm<128>(W_codes, g, sms, dev, s);
     return prompt::launch_gemm<64>(W_codes, g, sms, dev, s);

@@ -67,6 +67,28 @@ def test_prompt_matches_exact_value(rows, K, N, R, smooth, bias):
     assert st[0] == 0
 
 
+@pytest.mark.parametrize("rows,N,R", [(33, 136, 2), (40, 136, 96), (261, 1024, 66), (2049, 5120, 64)])      # (64-, 128- and 256-column tiles)
+def test_prompt_rows_behind_the_last_32_keep_fp32_z(rows, N, R):
+    """Ranks in pairs of opposite U signs whose z are large and equal but for one element of one pair: the output is twice that element. One
+    to eight rows behind the last whole 32 have z in full (a decode launch of as many rows has), so the output is right to a bf16
+    rounding and fp32 roundings of the large terms; of z as two bf16 parts 2^-17 could be missing, 1 % of these outputs."""
+    K = 4096
+    ops = BiLoCoLinear.synthetic(K, N, R, "cuda", seed=1).export_operands()
+    ops["W_codes"] = torch.zeros_like(ops["W_codes"])
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    V, U = torch.ones(R, K, device="cuda"), torch.ones(R, N, device="cuda")
+    V[R - 1, 1234] = -1.0
+    U[1::2] = -1.0
+    ops["V_packed"], ops["U_packed"] = kernel.pack_signs(V), kernel.pack_signs(U)
+    ops["S"] = torch.ones(R, device="cuda", dtype=torch.bfloat16)
+    x = (torch.rand(rows, K, device="cuda", generator=g) + 0.5).to(torch.bfloat16)
+    y = BiLoCoLinear.from_operands(ops)(x).double()
+    want = ((x.double() @ V.double().T) @ U.double())
+    last = slice(rows - rows % 32, rows)
+    err = (y - want)[last].abs()
+    assert bool((err <= want[last].abs() * 2.0 ** -9 + 4 * 4096 * 1.5 * 2.0 ** -24).all()), float((err / want[last].abs()).max())
+
+
 @pytest.mark.parametrize("R", [0, 32])
 def test_prompt_with_a_nan(R):
     """One NaN element: the tensor scale is what fp4.activation_scale_from_amax makes of a NaN maximum (1); rows without a NaN have the
