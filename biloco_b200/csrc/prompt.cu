@@ -148,7 +148,11 @@ __global__ void __launch_bounds__(Q_THREADS) quant_kernel(const __nv_bfloat16* _
 #pragma unroll
     for (int i = 1; i < Q_THREADS / 32; ++i) m = qm::max_nan(m, red[i]);
     const float gs = m > 0.f ? __fdiv_rn(m, 6.0f * target) : 1.0f;
-    if (blockIdx.x == 0 && threadIdx.x == 0) alpha_out[0] = __fmul_rn(w_gscale[0], gs);
+    // An alpha that underflows to zero leaves the low-rank term alone: zero codes, and 1 as the factor that z is divided by and the
+    // accumulator multiplied with.
+    const float alpha = __fmul_rn(w_gscale[0], gs);
+    const bool lr_alone = alpha == 0.f;
+    if (blockIdx.x == 0 && threadIdx.x == 0) alpha_out[0] = lr_alone ? 1.0f : alpha;
     const int kb_row = K >> 4, nkt = K >> 8;
     const long long total = (long long)rows * kb_row, stride = (long long)gridDim.x * Q_THREADS;
     for (long long i = (long long)blockIdx.x * Q_THREADS + threadIdx.x; i < total; i += stride) {
@@ -162,6 +166,7 @@ __global__ void __launch_bounds__(Q_THREADS) quant_kernel(const __nv_bfloat16* _
         uint2 c;
         uint8_t sf;
         qm::quant_block16<false>(x, gs, rule, c, sf);
+        if (lr_alone) { c = make_uint2(0u, 0u); sf = 0; }
         const int r = row & 127, b16 = kb & 15, ch = b16 >> 1;
         uint8_t* out = rec + ((size_t)(row >> 7) * nkt + (kb >> 4)) * A_REC;
         *reinterpret_cast<uint2*>(out + r * 128 + ((ch ^ (r & 7)) << 4) + (b16 & 1) * 8) = c;
@@ -374,7 +379,7 @@ __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__
                 float a = 0.f;
                 for (int src = 0; src < p.cs; ++src) a = __fadd_rn(a, part_sums[(src * W + 4 * j + i) * TM + row]);
                 float z = 0.f;
-                if (rank + i < p.R && alpha != 0.f) z = __fdiv_rn(__fmul_rn(a, __bfloat162float(p.S[rank + i])), alpha);
+                if (rank + i < p.R) z = __fdiv_rn(__fmul_rn(a, __bfloat162float(p.S[rank + i])), alpha);
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {            // (the remainders are exact; an infinity has none)
                     if (k == 2 && !third) break;

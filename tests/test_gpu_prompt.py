@@ -89,6 +89,26 @@ def test_prompt_rows_behind_the_last_32_keep_fp32_z(rows, N, R):
     assert bool((err <= want[last].abs() * 2.0 ** -9 + 4 * 4096 * 1.5 * 2.0 ** -24).all()), float((err / want[last].abs()).max())
 
 
+@pytest.mark.parametrize("wscale,xscale", [(1e-38, 1e-6), (0.0, 1.0), (1e-30, 1e-6), (1e-3, 1e-36)])
+def test_prompt_with_a_vanishing_alpha(wscale, xscale):
+    """alpha = w_gscale * activation scale underflows to zero, or is subnormal, or small with small activations: the low-rank term stays
+    (z is kept divided by alpha inside)."""
+    rows, K, N, R = 50, 512, 136, 96
+    ops = BiLoCoLinear.synthetic(K, N, R, "cuda", seed=4).export_operands()
+    ops["w_gscale"] = torch.full((1,), wscale, device="cuda")
+    ops["S"] = torch.ones_like(ops["S"])
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = (torch.randn(rows, K, device="cuda", generator=g) * xscale).to(torch.bfloat16)
+    y = BiLoCoLinear.from_operands(ops)(x).double()
+    want = (x.double() @ kernel.unpack_signs(ops["V_packed"]).double().T) @ kernel.unpack_signs(ops["U_packed"]).double()
+    if wscale == 1e-3:                       # (here the NVFP4 part is not negligible)
+        p, sf, gs = fp4.quantize_nvfp4(x.float(), fp4.CONFIG_X)
+        alpha = ops["w_gscale"] * gs
+        one = torch.ones(1, device="cuda")
+        want = want + (fp4.dequantize_nvfp4(p, sf, one).double() @ fp4.dequantize_nvfp4(ops["W_codes"], ops["W_sf"], one).double().T) * alpha.double()
+    assert float(torch.linalg.norm(y - want) / torch.linalg.norm(want)) <= 2e-3       # (bf16 rounding)
+
+
 @pytest.mark.parametrize("R", [0, 32])
 def test_prompt_with_a_nan(R):
     """One NaN element: the tensor scale is what fp4.activation_scale_from_amax makes of a NaN maximum (1); rows without a NaN have the
