@@ -19,6 +19,7 @@
 // 384: 562 -> 469.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 
 #include "../../include/biloco_b200.h"
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) decode_attention_kernel(const _
     float q[HPC][16], acc[HPC][16], mx[HPC], l[HPC];
 #pragma unroll
     for (int h = 0; h < HPC; ++h) {
-        mx[h] = -1e30f;
+        mx[h] = -FLT_MAX;
         l[h] = 0.f;
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
@@ -180,18 +181,21 @@ __global__ void __launch_bounds__(AT_THREADS, 1) decode_attention_kernel(const _
             for (int u = 0; u < UNR; ++u)
 #pragma unroll
                 for (int h = 0; h < HPC; ++h) sc[u][h] += __shfl_xor_sync(0xffffffffu, sc[u][h], o);
-        bool rise = false;
+        bool rise = false;                           // (a score is scaled and rounded once: the largest has the weight 1 whatever its size)
 #pragma unroll
         for (int h = 0; h < HPC; ++h) {
 #pragma unroll
-            for (int u = 0; u < UNR; ++u) rise |= sc[u][h] * p.scale > mx[h];
+            for (int u = 0; u < UNR; ++u) {
+                sc[u][h] = __fmul_rn(sc[u][h], p.scale);
+                rise |= sc[u][h] > mx[h];
+            }
         }
         if (__any_sync(0xffffffffu, rise)) {
 #pragma unroll
             for (int h = 0; h < HPC; ++h) {
                 float nm = mx[h];
 #pragma unroll
-                for (int u = 0; u < UNR; ++u) nm = fmaxf(nm, sc[u][h] * p.scale);
+                for (int u = 0; u < UNR; ++u) nm = fmaxf(nm, sc[u][h]);
                 const float corr = exp2f(mx[h] - nm);
                 l[h] *= corr;
 #pragma unroll
@@ -203,7 +207,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) decode_attention_kernel(const _
         for (int u = 0; u < UNR; ++u)
 #pragma unroll
             for (int h = 0; h < HPC; ++h) {
-                const float w = exp2f(fmaf(sc[u][h], p.scale, -mx[h]));
+                const float w = exp2f(__fsub_rn(sc[u][h], mx[h]));
                 l[h] += w;
 #pragma unroll
                 for (int e = 0; e < 16; ++e) acc[h][e] = fmaf(w, v[u][e], acc[h][e]);
@@ -234,7 +238,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) decode_attention_kernel(const _
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) v[u][e] = v_s[(e >> 3) * (D / 2) + sl * 8 + (e & 7)];
+            for (int e = 0; e < 16; ++e) v[u][e] = u == 0 && slot == 0 ? v_s[(e >> 3) * (D / 2) + sl * 8 + (e & 7)] : 0.f;      // (0 * an infinity is no zero)
 #pragma unroll
             for (int h = 0; h < HPC; ++h) {
                 float d = 0.f;
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) decode_attention_kernel(const _
     if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     for (int i = tid; i < HPC * D; i += AT_THREADS) {
         const int h = i / D, d = i - h * D;
-        float gm = -1e30f, num = 0.f, den = 0.f;
+        float gm = -FLT_MAX, num = 0.f, den = 0.f;
 #pragma unroll
         for (int w = 0; w < AT_WARPS; ++w) gm = fmaxf(gm, w_m[w][h]);
 #pragma unroll
@@ -284,7 +288,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) decode_attention_kernel(const _
     if (rank != 0) return;
     for (int i = tid; i < HPC * D; i += AT_THREADS) {
         const int h = i / D, d = i - h * D;
-        float gm = -1e30f, num = 0.f, den = 0.f;
+        float gm = -FLT_MAX, num = 0.f, den = 0.f;
         for (int r = 0; r < S; ++r) gm = fmaxf(gm, c_m[r][h]);
         for (int r = 0; r < S; ++r) {
             const float f = exp2f(c_m[r][h] - gm);

@@ -126,6 +126,67 @@ def test_attention_step_kernel_matches_torch_composition(M, H, KVH, D, qk_norm):
         cb["kv"][0][0][:, :, t] = ca["kv"][0][0][:, :, t]     # keep the two caches identical for the next position
 
 
+def _attention(qkv, kc, vc, pos, H, KVH, D):
+    """biloco_b200_decode_attention without norms, rotation by the angle zero."""
+    from biloco_b200 import _lib
+    M, L = qkv.shape[0], kc.shape[2]
+    cos, sin = torch.ones(L, D // 2, device="cuda"), torch.zeros(L, D // 2, device="cuda")
+    out = torch.empty(M, H * D, device="cuda", dtype=torch.bfloat16)
+    p = torch.tensor([pos], device="cuda")
+    _lib.check(_lib.load().biloco_b200_decode_attention(qkv.data_ptr(), None, None, 1e-6, cos.data_ptr(), sin.data_ptr(), p.data_ptr(), kc.data_ptr(), vc.data_ptr(),
+                                                        out.data_ptr(), M, H, KVH, D, L, torch.cuda.current_stream().cuda_stream), "decode_attention")
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,H,KVH,D,L", [(1, 32, 8, 128, 1000), (2, 6, 2, 64, 3000), (1, 8, 8, 64, 700), (3, 4, 1, 128, 200), (8, 32, 8, 128, 520), (1, 2, 1, 64, 66)])
+def test_attention_over_split_positions(M, H, KVH, D, L):
+    """Contexts long enough that a cluster shares the positions (more than 64 per CTA): the last position, ranges that are empty, of one
+    position, ragged; heads of 64 and 128, one, two and four query heads per CTA. Against float64; the output is bf16 (2^-9 of a
+    value) of fp32 sums over fp32 weights."""
+    g = torch.Generator(device="cuda").manual_seed(L)
+    kc = torch.randn(M, KVH, L, D, device="cuda", generator=g).to(torch.bfloat16)
+    vc = torch.randn(M, KVH, L, D, device="cuda", generator=g).to(torch.bfloat16)
+    kc[:, :, L // 3] *= 3.0                  # (a maximum that one CTA of the cluster has)
+    for pos in sorted({0, 1, 5, 63, 64, L // 2, L - 2, L - 1}):
+        qkv = torch.randn(M, (H + 2 * KVH) * D, device="cuda", generator=g).to(torch.bfloat16)
+        k, v = kc.clone(), vc.clone()
+        out = _attention(qkv, k, v, pos, H, KVH, D)
+        again = _attention(qkv, k, v, pos, H, KVH, D)
+        q, nk, nv = (t.view(M, -1, D) for t in qkv.split([H * D, KVH * D, KVH * D], dim=-1))
+        assert torch.equal(k[:, :, pos], nk) and torch.equal(v[:, :, pos], nv) and torch.equal(out, again)
+        keys = k[:, :, : pos + 1].double().repeat_interleave(H // KVH, 1)
+        vals = v[:, :, : pos + 1].double().repeat_interleave(H // KVH, 1)
+        w = torch.softmax((q.double().unsqueeze(2) @ keys.transpose(2, 3)) / D ** 0.5, dim=-1)
+        want = (w @ vals).reshape(M, H * D)
+        err = (out.double() - want).abs()
+        assert bool((err <= 2.0 ** -8 * want.abs() + 1e-5).all()), (pos, float(err.max()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [40, 1000])
+def test_attention_with_infinite_values_and_huge_scores(L):
+    """An infinite value element makes its column infinite and no other; scores of any finite size have a softmax (all equal: the mean)."""
+    H, KVH, D, pos = 4, 1, 128, 37
+    g = torch.Generator(device="cuda").manual_seed(1)
+    kc = torch.randn(1, KVH, L, D, device="cuda", generator=g).to(torch.bfloat16)
+    vc = torch.randn(1, KVH, L, D, device="cuda", generator=g).to(torch.bfloat16)
+    qkv = torch.randn(1, (H + 2 * KVH) * D, device="cuda", generator=g).to(torch.bfloat16)
+    inf = qkv.clone()
+    inf[0, (H + KVH) * D + 9] = float("inf")
+    out = _attention(inf, kc.clone(), vc.clone(), pos, H, KVH, D).view(H, D)
+    assert bool((out[:, 9] == float("inf")).all()) and bool(out[:, torch.arange(D, device="cuda") != 9].isfinite().all())
+    for size in (1e4, 1e16, -1e16):          # scores of size^2 sqrt(D), either sign
+        same = qkv.clone()
+        same[0, : H * D] = abs(size)
+        same[0, H * D:(H + KVH) * D] = size
+        k = torch.full_like(kc, size)
+        v = vc.clone()
+        out = _attention(same, k, v, pos, H, KVH, D).view(H, D).double()
+        want = v[0, 0, : pos + 1].double().mean(0)
+        assert bool(((out - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()), size
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,K,smooth", [(1, 9728, False), (8, 512, True), (32, 1024, False)])
 def test_swiglu_quantiser_and_fused_residual(M, K, smooth):
