@@ -48,7 +48,8 @@ struct QParams {
     uint8_t *codes, *sf, *rec;
     float *a_gscale, *alpha;
     const float* w_gscale;
-    int M, K, rule, given_scale, n_alpha;
+    int M, A_rows, K, rule, given_scale, n_alpha;
+    int pad;                             // the zero padding is written too
     int csize, gpc, seg, per, rpg;       // CTAs, groups per CTA, groups per row, vectors per segment, rows per group
     int staged;                          // the group's share fits shared memory; otherwise it is read from global memory again
     float eps, target;
@@ -267,6 +268,30 @@ __global__ void __launch_bounds__(GROUP * MAX_GPC) act_quant_kernel(const __grid
             }
         }
     }
+    // ---- zero padding, 16 bytes at a time: block scales of rows M .. 127 (a 16-byte chunk of an atom holds rows r, r + 32, r + 64,
+    //      r + 96), codes of rows M .. A_rows, the record's rest ----
+    if (p.pad) {
+        const int nth = p.csize * blockDim.x, at = crank * blockDim.x + tid;
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        auto pad_chunk = [&](uint8_t* atom, int r) {         // chunk r of an atom
+            if (r >= p.M && ((uintptr_t)atom & 15) == 0) *reinterpret_cast<uint4*>(atom + r * 16) = zero;
+            else
+                for (int q = 0; q < 4; ++q)
+                    if (r + 32 * q >= p.M) *reinterpret_cast<uint32_t*>(atom + r * 16 + q * 4) = 0u;
+        };
+        for (int i = at; i < kg * 32; i += nth) pad_chunk(p.sf + (size_t)(i >> 5) * 512, i & 31);
+        const long long ncode = (long long)(p.A_rows - p.M) * (p.K >> 4);
+        uint2* cz = reinterpret_cast<uint2*>(p.codes + (size_t)p.M * (p.K >> 1));
+        for (long long i = at; i < ncode; i += nth) cz[i] = make_uint2(0u, 0u);
+        if (p.rec) {
+            for (int i = at; i < kg * 32; i += nth) pad_chunk(p.rec + (size_t)(i >> 7) * rec_bytes + mma_n * 128 + ((i >> 5) & 3) * 512, i & 31);
+            const int tile = (mma_n - p.M) * 8;              // 16-byte chunks of a tile's rows M .. mma_n - 1
+            for (int i = at; i < (p.K >> 8) * tile; i += nth) {
+                const int kt = i / tile, c = i - kt * tile;
+                *reinterpret_cast<uint4*>(p.rec + (size_t)kt * rec_bytes + p.M * 128 + c * 16) = zero;
+            }
+        }
+    }
 }
 
 template <int PRO>
@@ -327,21 +352,13 @@ static int launch_act_quant(const void* X_bf16, const void* norm_w, float eps, c
     cudaStream_t s = (cudaStream_t)stream;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return BILOCO_ERR_CUDA;
-    // Zero padding -- block scales of rows M .. 127 of the last 128, codes of rows M .. A_rows, the record's rest -- is written only
-    // into buffers that do not have it yet (BILOCO_RULE_PADDED: outputs of an earlier call of the same shape).
-    if (!padded) {
-        const size_t sf_bytes = (size_t)((A_rows + 127) & ~127) * (K >> 4);
-        const size_t rec_bytes = A_rec ? (size_t)(K / 256) * ((M <= 8 ? 8 : (M <= 16 ? 16 : 32)) * 128 + 2048) : 0;
-        if (cudaMemsetAsync(A_sf, 0, sf_bytes, s) != cudaSuccess) return BILOCO_ERR_CUDA;
-        if (A_rows > M && cudaMemsetAsync((uint8_t*)A_codes + (size_t)M * (K >> 1), 0, (size_t)(A_rows - M) * (K >> 1), s) != cudaSuccess) return BILOCO_ERR_CUDA;
-        if (rec_bytes && cudaMemsetAsync(A_rec, 0, rec_bytes, s) != cudaSuccess) return BILOCO_ERR_CUDA;
-    }
     QParams p;
     p.X = (const __nv_bfloat16*)X_bf16; p.norm_w = (const __nv_bfloat16*)norm_w; p.smooth = (const __nv_bfloat16*)smooth_bf16;
     p.Xs = (__nv_bfloat16*)Xs_bf16;
     p.codes = (uint8_t*)A_codes; p.sf = (uint8_t*)A_sf; p.rec = (uint8_t*)A_rec;
     p.a_gscale = a_gscale; p.alpha = alpha_out; p.w_gscale = w_gscale;
-    p.M = M; p.K = K; p.rule = rule; p.given_scale = given_scale ? 1 : 0; p.n_alpha = n_alpha;
+    p.M = M; p.A_rows = A_rows; p.K = K; p.rule = rule; p.pad = padded ? 0 : 1;      // (BILOCO_RULE_PADDED: outputs of an earlier call of the same shape)
+    p.given_scale = given_scale ? 1 : 0; p.n_alpha = n_alpha;
     p.eps = eps; p.target = rule == BILOCO_RULE_STATIC_6 ? 448.0f : 256.0f;
     // groups: about one vector of 8 elements per thread, up to two groups in each of sixteen CTAs
     const int nv = K >> 3;

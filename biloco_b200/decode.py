@@ -160,7 +160,7 @@ class Decoder(nn.Module):
             st = dict(w_gs=torch.cat([l.w_gscale.reshape(1) for l in layers]).contiguous(), q=None)
             self._shared[(key, M)] = st
         q = fp4.quantize_activation(h.contiguous(), fp4.CONFIG_X, w_gscale=st["w_gs"], rows=M, out=st["q"],
-                                    norm_weight=norm_w, eps=self.c.eps)
+                                    norm_weight=norm_w, eps=self.c.eps, _padded=True)
         st["q"] = q
         if self.fuse_groups and 2 <= len(layers) <= 4 and "grouped" not in st:
             from .kernel import GroupedBiLoCoGemm

@@ -182,7 +182,7 @@ def _rec_buffer(M: int, K: int, dev):
 
 def quantize_activation(x: torch.Tensor, rule: str = None, smooth: torch.Tensor = None, w_gscale: torch.Tensor = None,
                         rows: int = None, out: dict = None, gscale: torch.Tensor = None, norm_weight: torch.Tensor = None,
-                        eps: float = 1e-6, swiglu: bool = False):
+                        eps: float = 1e-6, swiglu: bool = False, _padded: bool = False):
     """bf16 CUDA activation [M, K] -> dict(A [1, rows, K/2] uint8, A_sf float8 (atom layout), A_rec (the same codes and
     scales as the fused kernel stages them, or None), gscale fp32 [1],
     alpha fp32 [1] (= w_gscale * gscale, when w_gscale is given), X bf16 [M, K] (x / smooth when smoothing)).
@@ -193,7 +193,8 @@ def quantize_activation(x: torch.Tensor, rule: str = None, smooth: torch.Tensor 
     the same launch; X is then the normalised activation. ``w_gscale`` may hold n scales (fp32 [n]): alpha gets one entry
     per linear that consumes this activation.
     ``swiglu``: x is [M, 2K] = [gate | up] and the activation quantised is silu(gate) * up (each rounded to bf16, as the
-    separate torch kernels would), computed inside the same launch; X is that activation."""
+    separate torch kernels would), computed inside the same launch; X is that activation.
+    (``_padded``: `out` is the caller's own and only ever holds this shape, so its zero padding is in place.)"""
     rule_id = _lib.RULES[CONFIG_X if rule is None else rule]
     assert x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.is_contiguous()
     M, K = x.shape
@@ -211,7 +212,8 @@ def quantize_activation(x: torch.Tensor, rule: str = None, smooth: torch.Tensor 
                       if (smooth is not None or norm_weight is not None or swiglu) else x),
                    A_rec=_rec_buffer(M, K, dev))
     else:
-        rule_id |= 0x200            # (an earlier call of the same shape: its zero padding is in place)
+        if _padded:
+            rule_id |= 0x200
         if smooth is None and norm_weight is None and not swiglu:
             out["X"] = x
     if gscale is not None:          # tensor scale agreed elsewhere (tensor-parallel K-slices): do not recompute it

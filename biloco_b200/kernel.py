@@ -88,7 +88,7 @@ def tuned_mode(M: int, N: int, K: int, R: int, back_to_back: bool = True, device
             def run():
                 for gm in gemms:
                     if not back_to_back:
-                        fp4.quantize_activation(x, "mse", w_gscale=wgs, rows=M, out=q)
+                        fp4.quantize_activation(x, "mse", w_gscale=wgs, rows=M, out=q, _padded=True)
                     gm(q["A"], q["A_sf"], q["X"], A_rec=q.get("A_rec") if m != 7 else None)
             us = time_graph(run, None, iters=12, batch=1) / copies
             seen[m] = us

@@ -211,7 +211,7 @@ class BiLoCoLinear(nn.Module):
             if plan is not None and plan.smoothed is smoothed and plan.dev == x2.get_device():
                 return plan(x2, torch.empty((M, self.out_features), device=x2.device, dtype=torch.bfloat16), residual)
         q = fp4.quantize_activation(x2, fp4.CONFIG_X, smooth=self.smooth_scale if smoothed else None,
-                                    w_gscale=self.w_gscale, rows=M, out=self._acts.get((M, swiglu)), swiglu=swiglu)
+                                    w_gscale=self.w_gscale, rows=M, out=self._acts.get((M, swiglu)), swiglu=swiglu, _padded=True)
         self._acts[(M, swiglu)] = q
         g = self._gemm_for(M, q["alpha"])
         if not swiglu and x2.is_cuda:

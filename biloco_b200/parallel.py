@@ -209,7 +209,7 @@ class ShardedBiLoCoLinear:
         if self.kind == "row" and not self.local_scale:
             gscale = agree_on_activation_scale(x, smooth, group=self.group)
         q = fp4.quantize_activation(x, smooth=smooth, w_gscale=o["w_gscale"], rows=self.M, out=self._act.get(swiglu), gscale=gscale,
-                                    swiglu=swiglu)
+                                    swiglu=swiglu, _padded=True)
         self._act[swiglu] = q
         self.gemm.alpha = q["alpha"]
         if residual is not None:

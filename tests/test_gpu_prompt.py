@@ -228,3 +228,28 @@ def test_activation_quantiser_leaves_nan_elements_out(M, K, rule):
     live = s.view(torch.float8_e4m3fn).float().repeat_interleave(16, 1) * gs > 0
     want = torch.where(nan, torch.where((bits < 0) & live, 8, 0).to(torch.uint8), want)
     assert torch.equal(codes(q["A"][0]), want)
+
+
+@pytest.mark.parametrize("K,rows", [(512, 8), (2560, 32), (64, 128), (320, 40)])
+def test_activation_buffers_are_padded_again(K, rows):
+    """Buffers of an earlier call with more rows, or with anything in them: everything beyond the rows of this call is zero, in the codes, the
+    scale atoms and the record (which equals that of fresh buffers)."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    big = torch.randn(min(rows, 32), K, device="cuda", generator=g).to(torch.bfloat16)
+    q = fp4.quantize_activation(big, "mse", rows=rows)
+    for M in (big.shape[0] - 3, 1, big.shape[0]):
+        x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+        if M == 1:
+            q["A"].random_(0, 256, generator=g)
+            q["A_sf"].view(torch.uint8).random_(0, 256, generator=g)
+            if q["A_rec"] is not None:
+                q["A_rec"].random_(0, 256, generator=g)
+        if q["A_rec"] is not None and _lib.load().biloco_b200_act_rec_bytes(M, K) != q["A_rec"].numel():
+            q["A_rec"] = None                # (another record form)
+        q = fp4.quantize_activation(x, "mse", rows=rows, out=q)
+        p, sf, _ = fp4.quantize_nvfp4(x.float(), "mse")
+        assert torch.equal(q["A"][0, :M], p) and not bool(q["A"][0, M:].any())
+        assert torch.equal(q["A_sf"].view(torch.uint8), sf.view(torch.uint8))
+        fresh = fp4.quantize_activation(x, "mse", rows=rows)
+        if q["A_rec"] is not None:
+            assert torch.equal(q["A_rec"], fresh["A_rec"])
