@@ -108,7 +108,8 @@ def quantize_nvfp4(x: torch.Tensor, rule: str = None, global_scale=None):
     x = x.to(torch.float32)
     rows, K = x.shape
     if x.is_cuda and rows > 0 and K > 0:
-        return _quantize_nvfp4_cuda(x.contiguous(), rule, global_scale)
+        x = x.contiguous()
+        return _quantize_nvfp4_cuda(x if x.data_ptr() % 16 == 0 else x.clone(), rule, global_scale)      # (the kernels read 16 bytes at a time)
     return _quantize_nvfp4_torch(x, rule, global_scale)
 
 

@@ -67,6 +67,11 @@ def _raw_stream(dev):
     return torch._C._cuda_getCurrentRawStream(dev)
 
 
+def _aligned(t, n):
+    """t, or a copy of it where its memory does not start on n bytes."""
+    return t if t.data_ptr() % n == 0 else t.detach().clone()
+
+
 class BiLoCoLinear(nn.Module):
     def __init__(self, linear: nn.Linear, rank: int, method: str = "biloco", smooth_factor: float = 0.5):
         super().__init__()
@@ -256,12 +261,14 @@ class BiLoCoLinear(nn.Module):
             raise RuntimeError(f"fused linear does not support M={rows} N={N} K={K} R={R}")
         ws = torch.empty(nbytes, device=x2.device, dtype=torch.uint8)
         y = torch.empty((rows, N), device=x2.device, dtype=torch.bfloat16)
+        V = _aligned(self.V_packed, 8) if R else None         # (operands that are views into a larger buffer may start anywhere)
+        bias = _aligned(self.bias, 16) if self.bias is not None else None
         with torch.cuda.device(x2.device):
             rc = lib.biloco_b200_prompt_linear(
                 self.W_codes.data_ptr(), self.W_sf.data_ptr(), self.w_gscale.data_ptr(), x2.data_ptr(),
-                smooth.data_ptr() if smooth is not None else None, self.V_packed.data_ptr() if R else None,
+                smooth.data_ptr() if smooth is not None else None, V.data_ptr() if R else None,
                 self._ucol.data_ptr() if R else None, self.S.data_ptr() if R else None,
-                self.bias.data_ptr() if self.bias is not None else None, y.data_ptr(), ws.data_ptr(), nbytes, rows, N, K, R,
+                bias.data_ptr() if bias is not None else None, y.data_ptr(), ws.data_ptr(), nbytes, rows, N, K, R,
                 _lib.RULES[fp4.CONFIG_X], torch.cuda.current_stream().cuda_stream)
         _lib.check(rc, f"linear of {rows} rows (N={N}, K={K}, R={R})")
         return y

@@ -253,3 +253,24 @@ def test_activation_buffers_are_padded_again(K, rows):
         fresh = fp4.quantize_activation(x, "mse", rows=rows)
         if q["A_rec"] is not None:
             assert torch.equal(q["A_rec"], fresh["A_rec"])
+
+
+def test_operands_that_start_anywhere():
+    """Views that do not start on 16 bytes: a weight given to the quantiser, a prompt's bias and signs."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    flat = torch.randn(48 * 64 + 3, device="cuda", generator=g)
+    for off in (1, 2, 3):
+        W = flat[off:off + 48 * 64].view(48, 64)
+        for a, b in zip(fp4.quantize_nvfp4(W, "mse"), fp4.quantize_nvfp4(W.clone(), "mse")):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    K, N, R, rows = 512, 136, 40, 50
+    ops = BiLoCoLinear.synthetic(K, N, R, "cuda", seed=4).export_operands()
+    ops["bias"] = torch.randn(N, device="cuda", generator=g).to(torch.bfloat16)
+    x = torch.randn(rows, K, device="cuda", generator=g).to(torch.bfloat16)
+    want = BiLoCoLinear.from_operands(ops)(x)
+    odd = dict(ops)
+    odd["bias"] = torch.empty(N + 1, device="cuda", dtype=torch.bfloat16)[1:].copy_(ops["bias"])
+    odd["V_packed"] = torch.empty(R * K // 8 + 4, device="cuda", dtype=torch.uint8)[4:].view(R, K // 8).copy_(ops["V_packed"])
+    layer = BiLoCoLinear.from_operands(odd)
+    assert layer.bias.data_ptr() % 16 and layer.V_packed.data_ptr() % 8
+    assert torch.equal(layer(x), want)
