@@ -128,6 +128,31 @@ __global__ void __launch_bounds__(GROUP * MAX_GPC) act_quant_kernel(const __grid
     biloco::griddep_launch_dependents();                     // the consumer may start its own preamble (weight prefetch)
     if (p.csize > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // (every CTA runs before a peer writes to it)
     biloco::griddep_wait();                                  // nothing of the activation is read before the previous kernel has completed
+    const int kg = p.K >> 6, mma_n = p.M <= 8 ? 8 : (p.M <= 16 ? 16 : 32), rec_bytes = mma_n * 128 + 2048;
+    // ---- zero padding, 16 bytes at a time: block scales of rows M .. 127 (a 16-byte chunk of an atom holds rows r, r + 32, r + 64,
+    //      r + 96), codes of rows M .. A_rows, the record's rest ----
+    if (p.pad) {
+        const int nth = p.csize * blockDim.x, at = crank * blockDim.x + tid;
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        auto pad_chunk = [&](uint8_t* atom, int r) {         // chunk r of an atom
+            if (r >= p.M && ((uintptr_t)atom & 15) == 0) *reinterpret_cast<uint4*>(atom + r * 16) = zero;
+            else
+                for (int q = 0; q < 4; ++q)
+                    if (r + 32 * q >= p.M) *reinterpret_cast<uint32_t*>(atom + r * 16 + q * 4) = 0u;
+        };
+        for (int i = at; i < kg * 32; i += nth) pad_chunk(p.sf + (size_t)(i >> 5) * 512, i & 31);
+        const long long ncode = (long long)(p.A_rows - p.M) * (p.K >> 4);
+        uint2* cz = reinterpret_cast<uint2*>(p.codes + (size_t)p.M * (p.K >> 1));
+        for (long long i = at; i < ncode; i += nth) cz[i] = make_uint2(0u, 0u);
+        if (p.rec) {
+            for (int i = at; i < kg * 32; i += nth) pad_chunk(p.rec + (size_t)(i >> 7) * rec_bytes + mma_n * 128 + ((i >> 5) & 3) * 512, i & 31);
+            const int tile = (mma_n - p.M) * 8;              // 16-byte chunks of a tile's rows M .. mma_n - 1
+            for (int i = at; i < (p.K >> 8) * tile; i += nth) {
+                const int kt = i / tile, c = i - kt * tile;
+                *reinterpret_cast<uint4*>(p.rec + (size_t)kt * rec_bytes + p.M * 128 + c * 16) = zero;
+            }
+        }
+    }
     float amax = 0.f;
 #pragma unroll 1
     for (int r = 0; r < p.rpg; ++r) {
@@ -235,7 +260,6 @@ __global__ void __launch_bounds__(GROUP * MAX_GPC) act_quant_kernel(const __grid
             for (int i = 0; i < p.n_alpha; ++i) p.alpha[i] = __fmul_rn(p.w_gscale[i], gs);      // one per consumer of this activation
     }
     // ---- codes and scales (all lanes of a warp stay together: the block's two lanes exchange) ----
-    const int kg = p.K >> 6, mma_n = p.M <= 8 ? 8 : (p.M <= 16 ? 16 : 32), rec_bytes = mma_n * 128 + 2048;
 #pragma unroll 1
     for (int r = 0; r < nrows; ++r) {
         const int row = row0 + r;
@@ -265,30 +289,6 @@ __global__ void __launch_bounds__(GROUP * MAX_GPC) act_quant_kernel(const __grid
                 const int b = (i & 31) * 4;                  // byte of the word within the tile row
                 *reinterpret_cast<uint32_t*>(rk + row * 128 + (((b >> 4) ^ (row & 7)) << 4) + (b & 15)) = w;
                 if (!(lane & 1)) rk[mma_n * 128 + ((kb >> 2) & 3) * 512 + rsf + (kb & 3)] = sfb;
-            }
-        }
-    }
-    // ---- zero padding, 16 bytes at a time: block scales of rows M .. 127 (a 16-byte chunk of an atom holds rows r, r + 32, r + 64,
-    //      r + 96), codes of rows M .. A_rows, the record's rest ----
-    if (p.pad) {
-        const int nth = p.csize * blockDim.x, at = crank * blockDim.x + tid;
-        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-        auto pad_chunk = [&](uint8_t* atom, int r) {         // chunk r of an atom
-            if (r >= p.M && ((uintptr_t)atom & 15) == 0) *reinterpret_cast<uint4*>(atom + r * 16) = zero;
-            else
-                for (int q = 0; q < 4; ++q)
-                    if (r + 32 * q >= p.M) *reinterpret_cast<uint32_t*>(atom + r * 16 + q * 4) = 0u;
-        };
-        for (int i = at; i < kg * 32; i += nth) pad_chunk(p.sf + (size_t)(i >> 5) * 512, i & 31);
-        const long long ncode = (long long)(p.A_rows - p.M) * (p.K >> 4);
-        uint2* cz = reinterpret_cast<uint2*>(p.codes + (size_t)p.M * (p.K >> 1));
-        for (long long i = at; i < ncode; i += nth) cz[i] = make_uint2(0u, 0u);
-        if (p.rec) {
-            for (int i = at; i < kg * 32; i += nth) pad_chunk(p.rec + (size_t)(i >> 7) * rec_bytes + mma_n * 128 + ((i >> 5) & 3) * 512, i & 31);
-            const int tile = (mma_n - p.M) * 8;              // 16-byte chunks of a tile's rows M .. mma_n - 1
-            for (int i = at; i < (p.K >> 8) * tile; i += nth) {
-                const int kt = i / tile, c = i - kt * tile;
-                *reinterpret_cast<uint4*>(p.rec + (size_t)kt * rec_bytes + p.M * 128 + c * 16) = zero;
             }
         }
     }
