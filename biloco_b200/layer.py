@@ -28,6 +28,7 @@ class _DecodePlan:
         lib = _lib.load()
         self.keep = (layer.W_codes, layer.W_sf, layer.w_gscale, layer.smooth_scale, layer.V_packed, layer.S, q, g)
         self.g, self.smoothed, self.dev, self.N = g, layer.smoothed, q["A"].get_device(), layer.out_features
+        self._gs, self._sm = layer.w_gscale.data_ptr(), layer.smooth_scale.data_ptr()
         self.residual = g.residual if layer.bias is not None else None
         self._c = self.residual.data_ptr() if self.residual is not None else None
         R = layer.rank
@@ -42,6 +43,11 @@ class _DecodePlan:
                 q["alpha"].data_ptr(), g.V.data_ptr() if R else None, g.U_col32.data_ptr() if R else None, g.S.data_ptr() if R else None,
                 g.z.data_ptr(), g.z.numel() * 4, g.M, g.N, g.K, R, g.mode, ctypes.byref(h)), "layer_plan_create")
         self._h, self._run, self._destroy = h.value, lib.biloco_b200_layer_plan_run, lib.biloco_b200_layer_plan_destroy
+
+    def bound_to(self, layer):
+        """Whether the layer's scale and smoothing vector are still where the plan has them (a caller may replace these buffers)."""
+        b = layer._buffers
+        return self.smoothed is layer._smoothed and b["w_gscale"].data_ptr() == self._gs and b["smooth_scale"].data_ptr() == self._sm
 
     def __call__(self, x, y, residual=None):
         self.g.epoch += 1
@@ -213,7 +219,7 @@ class BiLoCoLinear(nn.Module):
         smoothed = self.smoothed
         if not swiglu:
             plan = self._plans.get(M)
-            if plan is not None and plan.smoothed is smoothed and plan.dev == x2.get_device():
+            if plan is not None and plan.dev == x2.get_device() and plan.bound_to(self):
                 return plan(x2, torch.empty((M, self.out_features), device=x2.device, dtype=torch.bfloat16), residual)
         q = fp4.quantize_activation(x2, fp4.CONFIG_X, smooth=self.smooth_scale if smoothed else None,
                                     w_gscale=self.w_gscale, rows=M, out=self._acts.get((M, swiglu)), swiglu=swiglu, _padded=True)
@@ -278,7 +284,7 @@ class BiLoCoLinear(nn.Module):
         K = self.in_features
         plan = self._plans.get(x.numel() // K)       # (a plan exists only for a quantised layer that has run at this batch)
         if (plan is not None and x.dtype is torch.bfloat16 and shape[-1] == K and plan.dev == x.get_device() and x.is_contiguous()
-                and plan.smoothed is self._smoothed):
+                and plan.bound_to(self)):
             return plan(x, x.new_empty(shape[:-1] + (self.out_features,)))
         assert self.weight is None, "call quantize() first"
         x2 = x.to(torch.bfloat16).reshape(-1, K).contiguous()

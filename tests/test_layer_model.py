@@ -178,3 +178,22 @@ def test_long_input_shares_one_tensor_scale_and_smoothed_follows_the_buffers():
     assert other.smoothed
     y2 = other(x[:8].contiguous()).float()
     assert torch.equal(y2, bl(x[:8].contiguous()).float())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 8, 40])
+def test_replaced_scale_and_smoothing_buffers_are_used(rows):
+    """w_gscale and smooth_scale are read on every call: assigned anew after a forward at this row count, the next one uses them."""
+    K, N, R = 512, 264, 40
+    ops = BiLoCoLinear.synthetic(K, N, R, "cuda", seed=4).export_operands()
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    ops["smooth_scale"] = (torch.rand(K, device="cuda", generator=g) + 0.5).to(torch.bfloat16)
+    x = torch.randn(rows, K, device="cuda", generator=g).to(torch.bfloat16)
+    layer = BiLoCoLinear.from_operands(ops)
+    for _ in range(2):
+        layer(x)
+    new = dict(ops, w_gscale=ops["w_gscale"] * 3, smooth_scale=(torch.rand(K, device="cuda", generator=g) + 0.5).to(torch.bfloat16))
+    layer.w_gscale, layer.smooth_scale = new["w_gscale"], new["smooth_scale"]
+    want = BiLoCoLinear.from_operands(new)(x)
+    for _ in range(2):
+        assert torch.equal(layer(x), want)
