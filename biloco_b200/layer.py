@@ -171,7 +171,13 @@ class BiLoCoLinear(nn.Module):
         self.W_sf.copy_(sf.view(torch.uint8))
         self.w_gscale.copy_(gs)
         self.weight = None
+        self._forget()
+
+    def _forget(self):
+        """Drop what was derived from the operands or from where they are (launchers with their re-laid copies, quantiser buffers, plans). A
+        CUDA graph captured over the layer holds addresses of these and has to be captured again."""
         self._gemms.clear()
+        self._acts.clear()
         self._plans.clear()
         self._ucol = None
 
@@ -191,7 +197,17 @@ class BiLoCoLinear(nn.Module):
     def _load_from_state_dict(self, *args, **kwargs):
         super()._load_from_state_dict(*args, **kwargs)
         self._smoothed = None
-        self._ucol = None
+        self._forget()
+
+    def _apply(self, fn, *args, **kwargs):
+        """(.to, .cuda, ...) Launchers and plans go where an operand has moved; a call that changes nothing leaves them."""
+        def where():
+            return [(t.data_ptr(), t.dtype) for t in (*self._buffers.values(), *self._parameters.values()) if t is not None]
+        before = where()
+        super()._apply(fn, *args, **kwargs)
+        if where() != before:
+            self._forget()
+        return self
 
     def export_operands(self):
         """What the fused kernel consumes, as a dict of tensors (the packed counterpart of the reference's state dict)."""

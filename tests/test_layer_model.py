@@ -197,3 +197,37 @@ def test_replaced_scale_and_smoothing_buffers_are_used(rows):
     want = BiLoCoLinear.from_operands(new)(x)
     for _ in range(2):
         assert torch.equal(layer(x), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("assign", [False, True])
+@pytest.mark.parametrize("bias", [False, True])
+def test_a_layer_that_has_run_takes_another_state(assign, bias):
+    """load_state_dict on a layer that has run at several row counts: every row count uses the new operands, also the re-laid copies of
+    them; the same after a move to the CPU and back. A .to() that changes nothing keeps the launchers."""
+    K, N, R = 512, 264, 40
+    g = torch.Generator(device="cuda").manual_seed(3)
+    xs = [torch.randn(m, K, device="cuda", generator=g).to(torch.bfloat16) for m in (1, 8, 40)]
+
+    def build(seed):
+        ops = BiLoCoLinear.synthetic(K, N, R, "cuda", seed=seed).export_operands()
+        ops["smooth_scale"] = (torch.rand(K, device="cuda", generator=g) + 0.5).to(torch.bfloat16)
+        if bias:
+            ops["bias"] = torch.randn(N, device="cuda", generator=g).to(torch.bfloat16)
+        return BiLoCoLinear.from_operands(ops)
+    a, b = build(1), build(2)
+    for x in xs + xs:
+        a(x)
+    kept = a._gemms[8]
+    a.to("cuda")
+    assert a._gemms[8] is kept
+    state = {k: v.clone() for k, v in b.state_dict().items()}
+    a.load_state_dict(state, assign=assign)
+    want = [b(x) for x in xs]
+    for _ in range(2):
+        for x, w in zip(xs, want):
+            assert torch.equal(a(x), w)
+    a.cpu()
+    a.cuda()
+    for x, w in zip(xs, want):
+        assert torch.equal(a(x), w)
