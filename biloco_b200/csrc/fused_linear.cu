@@ -769,7 +769,7 @@ extern "C" int biloco_b200_layer_plan_run(const void* plan, const void* X_bf16, 
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || (dev != q.dev && cudaSetDevice(q.dev) != cudaSuccess)) return BILOCO_ERR_CUDA;
     int rc = biloco_b200_norm_act_quant(X_bf16, nullptr, 0.f, q.smooth, q.Xs, q.A_codes, q.A_sf, q.A_rec, q.a_gscale, q.alpha, q.w_gscale, 1, q.M, q.M, q.K,
-                                        rule | BILOCO_RULE_PADDED, stream);      // (the first call of the layer at this batch padded them)
+                                        rule, stream);
     if (rc == BILOCO_OK)
         rc = fused_linear_impl(q.W_codes, q.W_sf, q.W_tiled, q.alpha, q.A_codes, q.A_sf, q.A_rec, q.smooth ? q.Xs : X_bf16, q.V, q.Ucol, q.S, C_bf16, Y,
                                q.scratch, q.scratch_bytes, q.M, q.M, q.N, q.K, q.R, q.mode, 1, stream);

@@ -181,6 +181,15 @@ def _rec_buffer(M: int, K: int, dev):
     return torch.empty(n, device=dev, dtype=torch.uint8) if n else None
 
 
+def _activation_buffers(M, rows, K, dev, n_alpha):
+    """What quantize_activation writes for M rows, padded to `rows` (all but X)."""
+    return dict(A=torch.empty((1, rows, K // 2), device=dev, dtype=torch.uint8),
+                A_sf=torch.empty(nvfp4_sf_bytes(rows, K), device=dev, dtype=torch.uint8).view(torch.float8_e4m3fn),
+                gscale=torch.empty(1, device=dev, dtype=torch.float32),
+                alpha=torch.empty(n_alpha, device=dev, dtype=torch.float32) if n_alpha else None,
+                X=None, A_rec=_rec_buffer(M, K, dev))
+
+
 def quantize_activation(x: torch.Tensor, rule: str = None, smooth: torch.Tensor = None, w_gscale: torch.Tensor = None,
                         rows: int = None, out: dict = None, gscale: torch.Tensor = None, norm_weight: torch.Tensor = None,
                         eps: float = 1e-6, swiglu: bool = False, _padded: bool = False):
@@ -205,13 +214,8 @@ def quantize_activation(x: torch.Tensor, rule: str = None, smooth: torch.Tensor 
     rows = M if rows is None else rows
     dev = x.device
     if out is None:
-        out = dict(A=torch.empty((1, rows, K // 2), device=dev, dtype=torch.uint8),
-                   A_sf=torch.empty(nvfp4_sf_bytes(rows, K), device=dev, dtype=torch.uint8).view(torch.float8_e4m3fn),
-                   gscale=torch.empty(1, device=dev, dtype=torch.float32),
-                   alpha=torch.empty(w_gscale.numel(), device=dev, dtype=torch.float32) if w_gscale is not None else None,
-                   X=(torch.empty((M, K), device=dev, dtype=torch.bfloat16)
-                      if (smooth is not None or norm_weight is not None or swiglu) else x),
-                   A_rec=_rec_buffer(M, K, dev))
+        out = _activation_buffers(M, rows, K, dev, w_gscale.numel() if w_gscale is not None else 0)
+        out["X"] = torch.empty((M, K), device=dev, dtype=torch.bfloat16) if (smooth is not None or norm_weight is not None or swiglu) else x
     else:
         if _padded:
             rule_id |= 0x200

@@ -28,6 +28,7 @@ class _DecodePlan:
         lib = _lib.load()
         self.keep = (layer.W_codes, layer.W_sf, layer.w_gscale, layer.smooth_scale, layer.V_packed, layer.S, q, g)
         self.g, self.smoothed, self.dev, self.N = g, layer.smoothed, q["A"].get_device(), layer.out_features
+        self._padded = 0
         self._gs, self._sm = layer.w_gscale.data_ptr(), layer.smooth_scale.data_ptr()
         self.residual = g.residual if layer.bias is not None else None
         self._c = self.residual.data_ptr() if self.residual is not None else None
@@ -51,8 +52,9 @@ class _DecodePlan:
 
     def __call__(self, x, y, residual=None):
         self.g.epoch += 1
-        rc = self._run(self._h, x.data_ptr(), self._c if residual is None else residual.data_ptr(), y.data_ptr(), _lib.RULES[fp4.CONFIG_X],
-                       _raw_stream(self.dev))
+        rc = self._run(self._h, x.data_ptr(), self._c if residual is None else residual.data_ptr(), y.data_ptr(),
+                       _lib.RULES[fp4.CONFIG_X] | self._padded, _raw_stream(self.dev))
+        self._padded = 0x200           # (BILOCO_RULE_PADDED: the first run has written the buffers' zero padding)
         if rc:
             _lib.check(rc, f"biloco linear (mode {self.g.mode}, M={self.g.M}, N={self.N}, K={self.g.K})")
         return y
@@ -231,18 +233,22 @@ class BiLoCoLinear(nn.Module):
         return g
 
     def _rows(self, x2, residual=None, swiglu=False):
-        M = x2.shape[0]
-        smoothed = self.smoothed
+        M, smoothed, dev = x2.shape[0], self.smoothed, x2.device
         if not swiglu:
+            assert x2.is_cuda, "the kernel forward needs CUDA tensors"
             plan = self._plans.get(M)
-            if plan is not None and plan.dev == x2.get_device() and plan.bound_to(self):
-                return plan(x2, torch.empty((M, self.out_features), device=x2.device, dtype=torch.bfloat16), residual)
+            if plan is None or plan.dev != x2.get_device() or not plan.bound_to(self):
+                q = self._acts.get((M, False))
+                if q is None or q["A"].device != dev or (smoothed and q["X"] is None):
+                    q = fp4._activation_buffers(M, M, self.in_features, dev, 1)
+                    q["X"] = torch.empty((M, self.in_features), device=dev, dtype=torch.bfloat16) if smoothed else None
+                    self._acts[(M, False)] = q
+                plan = self._plans[M] = _DecodePlan(self, q, self._gemm_for(M, q["alpha"]))
+            return plan(x2, torch.empty((M, self.out_features), device=dev, dtype=torch.bfloat16), residual)
         q = fp4.quantize_activation(x2, fp4.CONFIG_X, smooth=self.smooth_scale if smoothed else None,
-                                    w_gscale=self.w_gscale, rows=M, out=self._acts.get((M, swiglu)), swiglu=swiglu, _padded=True)
-        self._acts[(M, swiglu)] = q
+                                    w_gscale=self.w_gscale, rows=M, out=self._acts.get((M, True)), swiglu=True, _padded=True)
+        self._acts[(M, True)] = q
         g = self._gemm_for(M, q["alpha"])
-        if not swiglu and x2.is_cuda:
-            self._plans[M] = _DecodePlan(self, q, g)
         if self.bias is None:          # (with a bias, residual holds the broadcast bias)
             g.residual = residual
         return g(q["A"], q["A_sf"], q["X"], A_rec=q.get("A_rec")).view(-1, self.out_features)[:M]

@@ -208,7 +208,8 @@ int biloco_b200_fused_linear_act(const void* W_slab, const float* w_gscale, cons
  * biloco_b200_norm_act_quant (no norm) and biloco_b200_fused_linear_rec, kept by address -- they, the quantiser's outputs and
  * the scratch must outlive the plan; the plan belongs to the current device. run: the two launches for X bf16 [M, K] -> Y bf16
  * [M, N] (C bf16 [M, N] or NULL added before the rounding). Calls on one plan are ordered by the caller's stream, as launches that
- * share a scratch are. No counterpart in the reference (one Python forward per layer, biloco/layer.py:54-64). */
+ * share a scratch are. rule: as for the quantiser, with BILOCO_RULE_PADDED from the plan's second run on.
+ * No counterpart in the reference (one Python forward per layer, biloco/layer.py:54-64). */
 int biloco_b200_layer_plan_create(const void* W_codes, const void* W_sf, const void* W_tiled, const float* w_gscale, const void* smooth_bf16,
                                   void* Xs_bf16, void* A_codes, void* A_sf, void* A_rec, float* a_gscale, float* alpha, const void* V_packed,
                                   const int32_t* U_col32, const void* S_bf16, void* scratch, size_t scratch_bytes, int M, int N, int K, int R,
