@@ -70,8 +70,14 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {      // (exact: bf
 
 // Half a block per lane (lanes 2i and 2i + 1 hold one block): this lane's eight codes and, in both lanes, the block's scale.
 __device__ __forceinline__ uint32_t quant_half(const float (&x)[8], int lane, float gs, int rule, uint8_t& sf) {
-    uint32_t keep, sign;
-    float bmax = biloco::qm::half_max(x, keep, sign);
+    uint32_t keep = 0xffffffffu, sign = 0u;
+    float bmax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) bmax = biloco::qm::max_nan(bmax, fabsf(x[j]));
+    if (bmax != bmax) {
+        const biloco::qm::NanHalf n = biloco::qm::nan_half(x);
+        bmax = n.bmax; keep = n.keep; sign = n.sign;
+    }
     bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
     const float t = __fdiv_rn(bmax, gs);
     uint32_t c[2] = {0u, 0u};

@@ -112,23 +112,26 @@ __device__ __forceinline__ float max_nan(float a, float b) {
     return m;
 }
 
-// Largest |x_j| of half a block (NaN elements left out) and, for its codes, what a NaN element's code is: its sign bit over zero. The
-// conversion instructions would make it 6. `keep` has the other elements' nibbles, `sign` the NaN elements' sign bits.
-__device__ __forceinline__ float half_max(const float* x, uint32_t& keep, uint32_t& sign) {
-    float m = 0.f;
+// Half a block (eight bf16 values) that holds a NaN: the largest of the other elements, and what the conversion instructions would
+// make 6 -- the code of a NaN element is its sign bit over zero. `keep` has the other elements' nibbles, `sign` the NaN elements' sign
+// bits. Out of line: inlined, this rare path cost the prompt's quantiser 1.5 us at 96 rows of 5120.
+struct NanHalf { float bmax; uint32_t keep, sign; };
+static __device__ __noinline__ NanHalf nan_half(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+    NanHalf n = {0.f, 0xffffffffu, 0u};
+    const uint32_t w[4] = {w0, w1, w2, w3};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m = max_nan(m, fabsf(x[j]));
-    keep = 0xffffffffu;
-    sign = 0u;
-    if (m != m) {
-        m = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            m = fmaxf(m, fabsf(x[j]));
-            if (x[j] != x[j]) { keep &= ~(15u << (4 * j)); sign |= (__float_as_uint(x[j]) >> 31) << (4 * j + 3); }
-        }
+    for (int j = 0; j < 8; ++j) {
+        const float x = __uint_as_float((j & 1) ? w[j >> 1] & 0xFFFF0000u : w[j >> 1] << 16);
+        n.bmax = fmaxf(n.bmax, fabsf(x));
+        if (x != x) { n.keep &= ~(15u << (4 * j)); n.sign |= (__float_as_uint(x) >> 31) << (4 * j + 3); }
     }
-    return m;
+    return n;
+}
+__device__ __forceinline__ NanHalf nan_half(const float* x) {      // (bf16 values)
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w[e] = (__float_as_uint(x[2 * e]) >> 16) | (__float_as_uint(x[2 * e + 1]) & 0xFFFF0000u);
+    return nan_half(w[0], w[1], w[2], w[3]);
 }
 
 // Codes e2m1_rn(x_j / d) of half a block. The quotients are not formed: x_j times the reciprocal, made 2^-20 smaller and 2^-20
@@ -158,12 +161,12 @@ template <bool KEEP_NAN>
 __device__ __forceinline__ void quant_block16(const float (&x)[16], float gs, int rule, uint2& codes, uint8_t& sf) {
     float bmax = 0.f;
     uint32_t keep[2] = {0xffffffffu, 0xffffffffu}, sign[2] = {0u, 0u};
-    if constexpr (KEEP_NAN) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) bmax = max_nan(bmax, fabsf(x[j]));
-    } else {
-        bmax = half_max(x, keep[0], sign[0]);
-        bmax = fmaxf(bmax, half_max(x + 8, keep[1], sign[1]));
+    for (int j = 0; j < 16; ++j) bmax = max_nan(bmax, fabsf(x[j]));
+    if (!KEEP_NAN && bmax != bmax) {
+        const NanHalf l = nan_half(x), h = nan_half(x + 8);
+        bmax = fmaxf(l.bmax, h.bmax);
+        keep[0] = l.keep; keep[1] = h.keep; sign[0] = l.sign; sign[1] = h.sign;
     }
     float t = __fdiv_rn(bmax, gs);
     if (KEEP_NAN && t <= 0.f) t = 0.f;
