@@ -217,7 +217,8 @@ template <int NR> struct ZCfg {
     static_assert(ST * STAGE >= TM * NR * 4, "the exchange of the partial sums reuses the ring");
 };
 
-template <int NR>
+// THIRD: the last row tile gets third parts.
+template <int NR, bool THIRD>
 __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ ZParams p) {
     using C = ZCfg<NR>;
     extern __shared__ uint8_t smem_raw[];
@@ -381,11 +382,10 @@ __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__
                 float z = 0.f;
                 if (rank + i < p.R) z = __fdiv_rn(__fmul_rn(a, __bfloat162float(p.S[rank + i])), alpha);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {            // (the remainders are exact; an infinity has none)
-                    if (k == 2 && !third) break;
+                for (int k = 0; k < (THIRD ? 3 : 2); ++k) {          // (the remainders are exact; an infinity has none)
                     const __nv_bfloat16 h = __float2bfloat16_rn(z);
                     const uint32_t hb = __bfloat16_as_ushort(h);
-                    z = fabsf(__bfloat162float(h)) == INFINITY ? 0.f : z - __bfloat162float(h);
+                    z = THIRD && fabsf(__bfloat162float(h)) == INFINITY ? 0.f : z - __bfloat162float(h);
                     if (i & 1) part[k][i >> 1] |= hb << 16; else part[k][i >> 1] = hb;
                 }
             }
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__
                 uint8_t* o = p.zrec + ((size_t)rt * nlr + (rank >> 6)) * Z_REC + at;
                 *reinterpret_cast<uint2*>(o) = make_uint2(part[0][0], part[0][1]);
                 *reinterpret_cast<uint2*>(o + TM * 128) = make_uint2(part[1][0], part[1][1]);
-                if (third) *reinterpret_cast<uint2*>(p.z3 + (size_t)(rank >> 6) * (TM * 128) + at) = make_uint2(part[2][0], part[2][1]);
+                if (THIRD && third) *reinterpret_cast<uint2*>(p.z3 + (size_t)(rank >> 6) * (TM * 128) + at) = make_uint2(part[2][0], part[2][1]);
             }
         }
     }
@@ -742,11 +742,11 @@ struct Launch {
     }
 };
 
-template <int NR>
-static int launch_z(const CUtensorMap& tmX, ZParams z, int nrt, int sms, int dev, cudaStream_t s) {
+template <int NR, bool THIRD>
+static int launch_z_form(const CUtensorMap& tmX, ZParams z, int nrt, int sms, int dev, cudaStream_t s) {
     static bool ready[64] = {false};
     if (!ready[dev]) {
-        if (cudaFuncSetAttribute(z_gemm_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, ZCfg<NR>::SMEM) != cudaSuccess) return BILOCO_ERR_CUDA;
+        if (cudaFuncSetAttribute(z_gemm_kernel<NR, THIRD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ZCfg<NR>::SMEM) != cudaSuccess) return BILOCO_ERR_CUDA;
         ready[dev] = true;
     }
     z.ntr = (z.R + NR - 1) / NR;
@@ -754,7 +754,11 @@ static int launch_z(const CUtensorMap& tmX, ZParams z, int nrt, int sms, int dev
     z.cs = 1;
     while (z.cs < 8 && tiles * z.cs * 2 <= sms && (z.K >> 7) >= z.cs * 4) z.cs *= 2;
     Launch l(tiles * z.cs, Z_NT, ZCfg<NR>::SMEM, s, z.cs);
-    return cudaLaunchKernelEx(&l.cfg, z_gemm_kernel<NR>, tmX, z) == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
+    return cudaLaunchKernelEx(&l.cfg, z_gemm_kernel<NR, THIRD>, tmX, z) == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
+}
+template <int NR>
+static int launch_z(const CUtensorMap& tmX, const ZParams& z, int nrt, int sms, int dev, cudaStream_t s) {
+    return z.z3 ? launch_z_form<NR, true>(tmX, z, nrt, sms, dev, s) : launch_z_form<NR, false>(tmX, z, nrt, sms, dev, s);
 }
 
 template <int NT, bool THIRD>
