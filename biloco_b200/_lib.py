@@ -42,7 +42,7 @@ SIGNATURES = {
     "biloco_b200_layer_plan_run": (_i, [_vp] * 4 + [_i, _vp]),
     "biloco_b200_layer_plan_destroy": (_i, [_vp]),
     "biloco_b200_prompt_ws_bytes": (_sz, [_i] * 5),
-    "biloco_b200_prompt_linear": (_i, [_vp] * 11 + [_sz] + [_i] * 5 + [_vp]),
+    "biloco_b200_prompt_linear": (_i, [_vp] * 11 + [_sz, _vp] + [_i] * 5 + [_vp]),
     "biloco_b200_prompt_status": (_i, [ctypes.POINTER(ctypes.c_int32), _vp]),
     "biloco_b200_weight_quant_ws_bytes": (_sz, []),
     "biloco_b200_weight_quant": (_i, [_vp] * 5 + [_i] * 3 + [_vp]),

@@ -26,6 +26,7 @@
 
 extern "C" int biloco_internal_use_pdl();
 extern "C" unsigned long long biloco_internal_wait_ns();
+extern "C" int biloco_internal_skip_publish();
 extern "C" int biloco_internal_encode_map(void* map, int bf16, const void* ptr, int rows, int cols, int box_cols, int box_rows);
 
 namespace biloco {
@@ -41,13 +42,14 @@ constexpr int MMA_WARP = 9;
 constexpr int WPROD_WARP = 10;                   // GEMM only: the weights' copies, beside the activations' from PRODUCER_WARP
 constexpr int Z_NT = 320, G_NT = 352;            // threads of the z kernel and of the GEMM
 
-__device__ int32_t g_status[16];                 // first wait that ran out: code, CTA, kernel, role
+__device__ int32_t g_status[16];                 // the device's first wait that ran out since the last reading: code, CTA, kernel, role
 
 struct Ctrl {
     uint64_t full[8], empty[8], aux[8];
     uint64_t acc_full, acc_empty;
     uint32_t tmem_base;
     volatile int abort;
+    int32_t* status;                             // the caller's status words, or null
 };
 constexpr int CTRL_BYTES = 1024;
 static_assert(sizeof(Ctrl) <= CTRL_BYTES, "control block too large");
@@ -76,7 +78,8 @@ __device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, Ctrl* c, u
             if (t0 == 0) t0 = now;
             else if (now - t0 > ns) {
                 c->abort = 1;
-                if (atomicCAS(&g_status[0], 0, 120 + which) == 0) { g_status[1] = (int)blockIdx.x; g_status[2] = which; g_status[3] = role; }
+                for (int32_t* st : {g_status, c->status})
+                    if (st && atomicCAS(&st[0], 0, 120 + which) == 0) { st[1] = (int)blockIdx.x; st[2] = which; st[3] = role; }
                 return false;
             }
         }
@@ -207,6 +210,8 @@ struct ZParams {
     const __nv_bfloat16* S;
     const float* alpha;
     uint8_t *zrec, *z3;             // z3: third parts of the last row tile, or null
+    int32_t* status;
+    int skip;                       // test aid: this CTA's copies are left out (-1: none)
     unsigned long long wait_ns;
     int rows, K, R, nrt, ntr, cs;   // ntr: rank tiles
 };
@@ -237,6 +242,7 @@ __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__
         }
         mbar_init(smem_u32(&ctrl->acc_full), 1);
         ctrl->abort = 0;
+        ctrl->status = p.status;
         fence_mbar_init();
         prefetch_tmap(&tmX);
     }
@@ -248,7 +254,7 @@ __global__ void __launch_bounds__(Z_NT, 1) z_gemm_kernel(const __grid_constant__
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&ctrl->tmem_base);
     griddep_wait();
     if (warp == PRODUCER_WARP) {
-        if (lane == 0) {
+        if (lane == 0 && (int)blockIdx.x != p.skip) {
             fence_proxy_async_global();
             int s = 0;
             uint32_t par = 1u;
@@ -420,6 +426,8 @@ struct GParams {
     const float* alpha;
     const __nv_bfloat16* bias;
     __nv_bfloat16* Y;
+    int32_t* status;
+    int skip;                       // test aid: this CTA's copies are left out (-1: none)
     unsigned long long wait_ns;
     int rows, N, K, R, Rw, nrt, nnt, nlr;
 };
@@ -467,6 +475,7 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
         mbar_init(smem_u32(&ctrl->acc_full), 1);
         mbar_init(smem_u32(&ctrl->acc_empty), AUX_WARPS);
         ctrl->abort = 0;
+        ctrl->status = p.status;
         fence_mbar_init();
         prefetch_tmap(&tmW);
     }
@@ -480,7 +489,7 @@ __global__ void __launch_bounds__(G_NT, 1) gemm_kernel(const __grid_constant__ C
     if (warp == PRODUCER_WARP || warp == WPROD_WARP) {
         // Few and large copies: a wait-and-issue round of one thread takes about 370 cycles and 55 per further copy (measured), a
         // stage's MMAs 200 - 520. One warp brings the activation record (or z), the other the weight rows and their scales.
-        if (lane == 0) {
+        if (lane == 0 && (int)blockIdx.x != p.skip) {
             fence_proxy_async_global();
             int s = 0;
             uint32_t par = 1u;
@@ -801,7 +810,7 @@ extern "C" size_t biloco_b200_prompt_ws_bytes(int rows, int N, int K, int R, int
 
 extern "C" int biloco_b200_prompt_linear(const void* W_codes, const void* W_sf, const float* w_gscale, const void* X_bf16, const void* smooth_bf16,
                                          const void* V_packed, const int32_t* U_col32, const void* S_bf16, const void* bias_bf16, void* Y_bf16,
-                                         void* ws, size_t ws_bytes, int rows, int N, int K, int R, int rule, biloco_stream_t stream) {
+                                         void* ws, size_t ws_bytes, int32_t* status, int rows, int N, int K, int R, int rule, biloco_stream_t stream) {
     if (!W_codes || !W_sf || !w_gscale || !X_bf16 || !Y_bf16 || !ws) return BILOCO_ERR_NULL;
     if (R > 0 && (!V_packed || !U_col32 || !S_bf16)) return BILOCO_ERR_NULL;
     if (rule != BILOCO_RULE_STATIC_6 && rule != BILOCO_RULE_STATIC_4 && rule != BILOCO_RULE_MSE) return BILOCO_ERR_MODE;
@@ -809,7 +818,7 @@ extern "C" int biloco_b200_prompt_linear(const void* W_codes, const void* W_sf, 
     if (need == 0) return BILOCO_ERR_SHAPE;
     if (ws_bytes < need) return BILOCO_ERR_SCRATCH;
     if (((uintptr_t)W_codes & 15) || ((uintptr_t)W_sf & 15) || ((uintptr_t)X_bf16 & 15) || ((uintptr_t)smooth_bf16 & 15) || ((uintptr_t)bias_bf16 & 15) ||
-        ((uintptr_t)Y_bf16 & 15) || ((uintptr_t)ws & 255) || ((uintptr_t)V_packed & 7) || ((uintptr_t)U_col32 & 3))
+        ((uintptr_t)Y_bf16 & 15) || ((uintptr_t)ws & 255) || ((uintptr_t)V_packed & 7) || ((uintptr_t)U_col32 & 3) || ((uintptr_t)status & 3))
         return BILOCO_ERR_ALIGN;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -840,12 +849,12 @@ extern "C" int biloco_b200_prompt_linear(const void* W_codes, const void* W_sf, 
     if (R > 0) {
         CUtensorMap tmX;
         if (biloco_internal_encode_map(&tmX, 1, X, rows, K, 64, prompt::TM) != BILOCO_OK) return BILOCO_ERR_CUDA;
-        prompt::ZParams z = {(const uint8_t*)V_packed, (const __nv_bfloat16*)S_bf16, alpha, w + L.zrec, L.third ? w + L.z3 : nullptr, ns, rows, K, R, L.nrt, 0, 0};
+        prompt::ZParams z = {(const uint8_t*)V_packed, (const __nv_bfloat16*)S_bf16, alpha, w + L.zrec, L.third ? w + L.z3 : nullptr, status, biloco_internal_skip_publish(), ns, rows, K, R, L.nrt, 0, 0};
         // 128 ranks per tile halve the reads of X; 64 where that would leave the device half empty
         const int rc = (R > 64 && L.nrt * ((R + 127) / 128) * 8 >= sms) ? prompt::launch_z<128>(tmX, z, L.nrt, sms, dev, s) : prompt::launch_z<64>(tmX, z, L.nrt, sms, dev, s);
         if (rc != BILOCO_OK) return rc;
     }
-    prompt::GParams g = {w + L.arec, w + L.zrec, L.third ? w + L.z3 : nullptr, (const uint8_t*)W_sf, U_col32, alpha, (const __nv_bfloat16*)bias_bf16, (__nv_bfloat16*)Y_bf16, ns,
+    prompt::GParams g = {w + L.arec, w + L.zrec, L.third ? w + L.z3 : nullptr, (const uint8_t*)W_sf, U_col32, alpha, (const __nv_bfloat16*)bias_bf16, (__nv_bfloat16*)Y_bf16, status, biloco_internal_skip_publish(), ns,
                          rows, N, K, R, (R + 31) / 32, L.nrt, 0, L.nlr};
     const double c64 = prompt::gemm_cost(64, 50, L.nrt, N, K / 256, L.nlr, sms, L.third), c128 = prompt::gemm_cost(128, 66, L.nrt, N, K / 256, L.nlr, sms, L.third),
                  c256 = prompt::gemm_cost(256, 130, L.nrt, N, K / 256, L.nlr, sms, L.third);
@@ -854,9 +863,13 @@ extern "C" int biloco_b200_prompt_linear(const void* W_codes, const void* W_sf, 
     return prompt::launch_gemm<64>(W_codes, g, sms, dev, s);
 }
 
-// The status words of this device's prompt launches (synchronises): word 0 is non-zero after a device-side wait ran out.
+// The device's prompt launches since the last reading (synchronises, and clears): word 0 is non-zero if a device-side wait ran out.
 extern "C" int biloco_b200_prompt_status(int32_t* out16, biloco_stream_t stream) {
     if (!out16) return BILOCO_ERR_NULL;
-    if (cudaMemcpyFromSymbolAsync(out16, prompt::g_status, sizeof(int32_t) * 16, 0, cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess) return BILOCO_ERR_CUDA;
+    void* words = nullptr;
+    if (cudaGetSymbolAddress(&words, prompt::g_status) != cudaSuccess ||
+        cudaMemcpyAsync(out16, words, sizeof(int32_t) * 16, cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess ||
+        cudaMemsetAsync(words, 0, sizeof(int32_t) * 16, (cudaStream_t)stream) != cudaSuccess)
+        return BILOCO_ERR_CUDA;
     return cudaStreamSynchronize((cudaStream_t)stream) == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
 }

@@ -327,9 +327,12 @@ class _FP4Only:
         self.mode = _lib.MODE_COUNTER
         with torch.cuda.device(dev):
             nbytes = scratch_bytes(M, self.N, self.K, 0)
+            self._head = _lib.load().biloco_b200_scratch_head_bytes(M, self.N, self.K, 0, 0) // 4
         self.z = torch.zeros(nbytes // 4, device=dev, dtype=torch.float32)
         self.epoch = 0
         self.residual = None
+
+    reset, status = BiLoCoGemm.reset, BiLoCoGemm.status
 
     def __call__(self, A, A_sf, X_bf16=None, out=None, A_rec=None):
         self.epoch += 1

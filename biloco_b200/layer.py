@@ -105,6 +105,7 @@ class BiLoCoLinear(nn.Module):
         self._acts = {}       # (decode batch M, SwiGLU input?) -> reusable activation-quantiser outputs
         self._plans = {}      # decode batch M -> _DecodePlan
         self._ucol = None     # U signs by column, for more than MAX_ROWS rows (built on first use)
+        self._status = None   # status words of launches for more than MAX_ROWS rows
 
     @classmethod
     def synthetic(cls, in_features: int, out_features: int, rank: int, device, seed: int = 0):
@@ -126,7 +127,7 @@ class BiLoCoLinear(nn.Module):
         self.register_buffer("W_sf", sf.view(torch.uint8))
         self.register_buffer("w_gscale", torch.full((1,), 1e-3, device=device, dtype=torch.float32))
         self._smoothed = False
-        self._gemms, self._acts, self._plans, self._ucol = {}, {}, {}, None
+        self._gemms, self._acts, self._plans, self._ucol, self._status = {}, {}, {}, None, None
         return self
 
     @classmethod
@@ -144,7 +145,7 @@ class BiLoCoLinear(nn.Module):
             self.register_buffer(name, ops[name].contiguous())
         self.register_buffer("W_sf", ops["W_sf"].view(torch.uint8).contiguous())
         self._smoothed = None
-        self._gemms, self._acts, self._plans, self._ucol = {}, {}, {}, None
+        self._gemms, self._acts, self._plans, self._ucol, self._status = {}, {}, {}, None, None
         return self
 
     # ------------------------------------------------------------------------------------------------------
@@ -210,6 +211,19 @@ class BiLoCoLinear(nn.Module):
         if where() != before:
             self._forget()
         return self
+
+    def status(self):
+        """The first non-zero status words (synchronises; word 0: a device-side wait ran out, the output of that call is not whole) among the
+        layer's launches at every row count, or sixteen zeros."""
+        words = [g.status() for g in self._gemms.values()] + ([self._status.tolist()] if self._status is not None else [])
+        return next((w for w in words if w[0]), [0] * 16)
+
+    def reset_status(self):
+        """Clear the status words (and with a launcher's its scratch), after status() reported a wait."""
+        for g in self._gemms.values():
+            g.reset()
+        if self._status is not None:
+            self._status.zero_()
 
     def export_operands(self):
         """What the fused kernel consumes, as a dict of tensors (the packed counterpart of the reference's state dict)."""
@@ -284,6 +298,8 @@ class BiLoCoLinear(nn.Module):
         if R and self._ucol is None:
             from .kernel import pack_u_col32
             self._ucol = pack_u_col32(self.U_packed, N, R)
+        if self._status is None or self._status.device != x2.device:
+            self._status = torch.zeros(16, device=x2.device, dtype=torch.int32)
         nbytes = lib.biloco_b200_prompt_ws_bytes(rows, N, K, R, 0 if smooth is None else 1)
         if nbytes == 0:
             raise RuntimeError(f"fused linear does not support M={rows} N={N} K={K} R={R}")
@@ -296,7 +312,7 @@ class BiLoCoLinear(nn.Module):
                 self.W_codes.data_ptr(), self.W_sf.data_ptr(), self.w_gscale.data_ptr(), x2.data_ptr(),
                 smooth.data_ptr() if smooth is not None else None, V.data_ptr() if R else None,
                 self._ucol.data_ptr() if R else None, self.S.data_ptr() if R else None,
-                bias.data_ptr() if bias is not None else None, y.data_ptr(), ws.data_ptr(), nbytes, rows, N, K, R,
+                bias.data_ptr() if bias is not None else None, y.data_ptr(), ws.data_ptr(), nbytes, self._status.data_ptr(), rows, N, K, R,
                 _lib.RULES[fp4.CONFIG_X], torch.cuda.current_stream().cuda_stream)
         _lib.check(rc, f"linear of {rows} rows (N={N}, K={K}, R={R})")
         return y

@@ -231,12 +231,14 @@ int biloco_b200_weight_quant(const float* X, void* ws, void* codes, void* sf, fl
  * from the row-major weight codes and scale atoms. X bf16 [rows, K], smooth bf16 [K] or NULL, w_gscale fp32 [1], V_packed u8
  * [R, K/8], U_col32 int32 [N, ceil(R/32)], S bf16 [R], bias bf16 [N] or NULL, Y bf16 [rows, N]; R = 0: NVFP4 GEMM alone.
  * K a multiple of 256, N of 8. ws: biloco_b200_prompt_ws_bytes bytes, 256-byte aligned, need not be cleared or kept.
- * Waits are bounded as in the fused linear; biloco_b200_prompt_status reads (and synchronises) the device's status words.
+ * Waits are bounded as in the fused linear. After one that ran out rows of Y are unwritten and `status` (16 words, zeroed by the caller
+ * once, or NULL) holds what biloco_b200_read_status describes, until the caller clears it; biloco_b200_prompt_status reads and
+ * clears the same for all prompt launches of the current device (synchronises).
  * Replaces: BiLoCoLinear.forward of the reference on long inputs (biloco/layer.py:54-64). */
 size_t biloco_b200_prompt_ws_bytes(int rows, int N, int K, int R, int smooth);
 int biloco_b200_prompt_linear(const void* W_codes, const void* W_sf, const float* w_gscale, const void* X_bf16, const void* smooth_bf16,
                               const void* V_packed, const int32_t* U_col32, const void* S_bf16, const void* bias_bf16, void* Y_bf16,
-                              void* ws, size_t ws_bytes, int rows, int N, int K, int R, int rule, biloco_stream_t stream);
+                              void* ws, size_t ws_bytes, int32_t* status, int rows, int N, int K, int R, int rule, biloco_stream_t stream);
 int biloco_b200_prompt_status(int32_t* out16, biloco_stream_t stream);
 
 /* A_rec (optional, biloco_b200_act_rec_bytes(M, K) bytes, K % 256 == 0, M <= 32): the same codes and block scales once
@@ -423,7 +425,7 @@ int biloco_b200_read_status(const void* scratch, int32_t* out16, biloco_stream_t
  * Counterpart in the reference: the bounded polls that record codes in Diag[4095] (csrc/biloco_gemm.cu:1149-1151). */
 #define BILOCO_OPT_WAIT_BUDGET_US 5
 /* Test aid for the failure path: CTA `value` of a row-slab launch, or of a launch of schedules 2 and 4 from five rows,
- * computes its z values (partial sums of z) but does not publish them, so
+ * computes its z values (partial sums of z) but does not publish them, or of a prompt launch does not fetch its operands, so
  * that every consumer's poll runs out of its budget (-1, the default: off). */
 #define BILOCO_OPT_SKIP_PUBLISH 6
 /* Row-slab schedule: weight records a CTA keeps in flight while it fills its ring ahead of the dependency wait

@@ -101,6 +101,43 @@ def test_batch_z_poll_runs_out_and_later_launches_are_right(M):
     assert torch.equal(run(0).view(torch.int16), clean[0].view(torch.int16)) and g.status()[0] == 0
 
 
+@pytest.mark.parametrize("R", [0, 96])
+def test_prompt_wait_runs_out_and_the_layer_says_so(R):
+    """More than 32 rows: one CTA of the z launch and of the GEMM does not fetch its operands, its waits run out of the budget. The layer's
+    own status words say so until they are cleared, another layer's do not; the calls after it are right."""
+    import ctypes
+    from biloco_b200 import _lib
+    from biloco_b200.layer import BiLoCoLinear
+    lib = _lib.load()
+    K, N, rows = 1024, 264, 140
+    ops = BiLoCoLinear.synthetic(K, N, max(R, 1), "cuda", seed=4).export_operands()
+    if R == 0:
+        ops["V_packed"], ops["U_packed"], ops["S"] = ops["V_packed"][:0], ops["U_packed"][:0], ops["S"][:0]
+    layer, other = BiLoCoLinear.from_operands(ops), BiLoCoLinear.from_operands(ops)
+    x = torch.randn(rows, K, device="cuda").to(torch.bfloat16)
+    clean = layer(x)
+    assert torch.equal(other(x), clean) and layer.status() == [0] * 16
+    try:
+        lib.biloco_b200_set_option(_lib.OPT_WAIT_BUDGET_US, 2000)
+        lib.biloco_b200_set_option(_lib.OPT_SKIP_PUBLISH, 0)
+        t0 = time.perf_counter()
+        layer(x)
+        torch.cuda.synchronize()
+        dt = time.perf_counter() - t0
+    finally:
+        lib.biloco_b200_set_option(_lib.OPT_SKIP_PUBLISH, -1)
+        lib.biloco_b200_set_option(_lib.OPT_WAIT_BUDGET_US, 0)
+    st = layer.status()
+    assert st[0] in (121, 122) and st[1] == 0 and dt < 1.0, (st[:4], dt)
+    assert torch.equal(other(x), clean) and other.status() == [0] * 16
+    assert torch.equal(layer(x), clean) and layer.status()[0] == st[0]
+    layer.reset_status()
+    assert layer.status() == [0] * 16
+    words = (ctypes.c_int32 * 16)()
+    for want in (st[0], 0):                  # (the device-wide words: read and cleared)
+        assert lib.biloco_b200_prompt_status(words, torch.cuda.current_stream().cuda_stream) == 0 and words[0] == want
+
+
 def test_peer_allreduce_wait_runs_out_and_reports(lib):
     """The peer all-reduce polls its own receive buffer for the peers' words with a time budget. Here a 'group' of two
     with nobody behind rank 1 (its buffer is a second local allocation that nothing reads or writes back): the poll runs
