@@ -49,7 +49,6 @@ struct QParams {
     float *a_gscale, *alpha;
     const float* w_gscale;
     int M, A_rows, K, rule, given_scale, n_alpha;
-    int pad;                             // the zero padding is written too
     int csize, gpc, seg, per, rpg;       // CTAs, groups per CTA, groups per row, vectors per segment, rows per group
     int staged;                          // the group's share fits shared memory; otherwise it is read from global memory again
     float eps, target;
@@ -113,8 +112,9 @@ __device__ __forceinline__ uint32_t quant_half(const float (&x)[8], int lane, fl
     return four ? c[1] : c[0];
 }
 
-// PRO: 0 the activation as it is (or smoothed), 1 RMS norm in front, 2 silu(gate) * up in front
-template <int PRO>
+// PRO: 0 the activation as it is (or smoothed), 1 RMS norm in front, 2 silu(gate) * up in front. PAD: the zero padding is written too (a
+// form of its own: its code in the launches that skip it cost them 0.5 us: decode step of one sequence 434 -> 424).
+template <int PRO, bool PAD>
 __global__ void __launch_bounds__(GROUP * MAX_GPC) act_quant_kernel(const __grid_constant__ QParams p) {
     extern __shared__ uint4 stage_raw[];                     // [group][row][vector of the segment]
     __shared__ float red[GROUP * MAX_GPC / 32];
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(GROUP * MAX_GPC) act_quant_kernel(const __grid
     const int kg = p.K >> 6, mma_n = p.M <= 8 ? 8 : (p.M <= 16 ? 16 : 32), rec_bytes = mma_n * 128 + 2048;
     // ---- zero padding, 16 bytes at a time: block scales of rows M .. 127 (a 16-byte chunk of an atom holds rows r, r + 32, r + 64,
     //      r + 96), codes of rows M .. A_rows, the record's rest ----
-    if (p.pad) {
+    if constexpr (PAD) {
         const int nth = p.csize * blockDim.x, at = crank * blockDim.x + tid;
         const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
         auto pad_chunk = [&](uint8_t* atom, int r) {         // chunk r of an atom
@@ -300,16 +300,20 @@ __global__ void __launch_bounds__(GROUP * MAX_GPC) act_quant_kernel(const __grid
     }
 }
 
-template <int PRO>
-static cudaError_t launch_pro(cudaLaunchConfig_t* cfg, const QParams& p, int dev) {
+template <int PRO, bool PAD>
+static cudaError_t launch_form(cudaLaunchConfig_t* cfg, const QParams& p, int dev) {
     static bool ready[64] = {false};
     if (dev >= 0 && dev < 64 && !ready[dev]) {
-        cudaFuncSetAttribute(act_quant_kernel<PRO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        cudaFuncSetAttribute(act_quant_kernel<PRO>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaFuncSetAttribute(act_quant_kernel<PRO, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+        cudaFuncSetAttribute(act_quant_kernel<PRO, PAD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaGetLastError();
         ready[dev] = true;
     }
-    return cudaLaunchKernelEx(cfg, act_quant_kernel<PRO>, p);
+    return cudaLaunchKernelEx(cfg, act_quant_kernel<PRO, PAD>, p);
+}
+template <int PRO>
+static cudaError_t launch_pro(cudaLaunchConfig_t* cfg, const QParams& p, int dev, bool pad) {      // (pad: not with BILOCO_RULE_PADDED)
+    return pad ? launch_form<PRO, true>(cfg, p, dev) : launch_form<PRO, false>(cfg, p, dev);
 }
 
 // Whether the device takes a cluster of sixteen such CTAs (asked once per device; the answer depends on how its SMs are grouped).
@@ -329,9 +333,9 @@ static bool sixteen_fit(int dev) {
         cfg.dynamicSmemBytes = 96 * 1024;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        bool ok = cudaFuncSetAttribute(act_quant_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024) == cudaSuccess &&
-                  cudaFuncSetAttribute(act_quant_kernel<0>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                  cudaOccupancyMaxActiveClusters(&n, act_quant_kernel<0>, &cfg) == cudaSuccess && n >= 1;
+        bool ok = cudaFuncSetAttribute(act_quant_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024) == cudaSuccess &&
+                  cudaFuncSetAttribute(act_quant_kernel<0, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&n, act_quant_kernel<0, false>, &cfg) == cudaSuccess && n >= 1;
         cudaGetLastError();
         known[dev] = ok ? 1 : -1;
     }
@@ -363,8 +367,7 @@ static int launch_act_quant(const void* X_bf16, const void* norm_w, float eps, c
     p.Xs = (__nv_bfloat16*)Xs_bf16;
     p.codes = (uint8_t*)A_codes; p.sf = (uint8_t*)A_sf; p.rec = (uint8_t*)A_rec;
     p.a_gscale = a_gscale; p.alpha = alpha_out; p.w_gscale = w_gscale;
-    p.M = M; p.A_rows = A_rows; p.K = K; p.rule = rule; p.pad = padded ? 0 : 1;      // (BILOCO_RULE_PADDED: outputs of an earlier call of the same shape)
-    p.given_scale = given_scale ? 1 : 0; p.n_alpha = n_alpha;
+    p.M = M; p.A_rows = A_rows; p.K = K; p.rule = rule; p.given_scale = given_scale ? 1 : 0; p.n_alpha = n_alpha;
     p.eps = eps; p.target = rule == BILOCO_RULE_STATIC_6 ? 448.0f : 256.0f;
     // groups: about one vector of 8 elements per thread, up to two groups in each of sixteen CTAs
     const int nv = K >> 3;
@@ -400,7 +403,7 @@ static int launch_act_quant(const void* X_bf16, const void* norm_w, float eps, c
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    const cudaError_t e = norm_w ? launch_pro<1>(&cfg, p, dev) : (swiglu ? launch_pro<2>(&cfg, p, dev) : launch_pro<0>(&cfg, p, dev));
+    const cudaError_t e = norm_w ? launch_pro<1>(&cfg, p, dev, !padded) : (swiglu ? launch_pro<2>(&cfg, p, dev, !padded) : launch_pro<0>(&cfg, p, dev, !padded));
     return e == cudaSuccess ? BILOCO_OK : BILOCO_ERR_CUDA;
 }
 
