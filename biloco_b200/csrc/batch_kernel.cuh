@@ -573,41 +573,42 @@ __global__ void __launch_bounds__(NT, 1) batch_kernel(const __grid_constant__ CU
                             image_half(img + b * IMG, r128, half, uw[i]);
                         }
                     }
-                    // z pieces: thread = (row, 8 ranks of a chunk); polled until every value carries this launch's mark
-                    const int m = tid >> 3, pc = tid & 7;
+                    // z pieces: thread = (row, 8 ranks of a chunk), the chunks of a batch over the groups of MMA_N * 8 threads there are (four at 8
+                    // rows: splitting z into three parts by one group after another was 20 us of 600 in the decode step of eight sequences);
+                    // polled until every value carries this launch's mark
+                    constexpr int ZT = MMA_N * 8 < EPI_THREADS ? MMA_N * 8 : EPI_THREADS;
+                    const int m = (tid & (ZT - 1)) >> 3, pc = tid & 7;
 #pragma unroll 1
-                    for (int i = 0; i < nr; ++i) {
+                    for (int i = tid / ZT; i < nr; i += EPI_THREADS / ZT) {
                         const int b = (ib + i) & (NIMG - 1), w = w0 + 2 * (cb + i) + (pc >> 2), e0 = 32 * (w0 + 2 * (cb + i)) + 8 * pc;
-                        if (tid < MMA_N * 8) {
-                            uint32_t part[CF::PARTS][4];
+                        uint32_t part[CF::PARTS][4];
 #pragma unroll
-                            for (int k = 0; k < CF::PARTS; ++k) part[k][0] = part[k][1] = part[k][2] = part[k][3] = 0u;
-                            if (m < p.M && w < w1 && e0 < p.Rg) {
-                                const float* src = zb + (size_t)m * p.Rpad + e0;
-                                uint32_t v[8];
-                                Poll poll;
+                        for (int k = 0; k < CF::PARTS; ++k) part[k][0] = part[k][1] = part[k][2] = part[k][3] = 0u;
+                        if (m < p.M && w < w1 && e0 < p.Rg) {
+                            const float* src = zb + (size_t)m * p.Rpad + e0;
+                            uint32_t v[8];
+                            Poll poll;
 #pragma unroll 1
-                                while (true) {
-                                    const uint4 a = ld_volatile_v4(src), c = ld_volatile_v4(src + 4);
-                                    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
-                                    uint32_t bad = 0u;
+                            while (true) {
+                                const uint4 a = ld_volatile_v4(src), c = ld_volatile_v4(src + 4);
+                                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+                                uint32_t bad = 0u;
 #pragma unroll
-                                    for (int q = 0; q < 8; ++q) bad |= (e0 + q < p.Rg) ? (v[q] ^ phase) : 0u;
-                                    if (!(bad & 1u)) break;
-                                    if (poll.expired(ctrl, p, ST_Z)) break;
-                                }
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) {
-                                    float z0 = e0 + 2 * q < p.Rg ? unmark(v[2 * q]) : 0.f, z1 = e0 + 2 * q + 1 < p.Rg ? unmark(v[2 * q + 1]) : 0.f;
-#pragma unroll
-                                    for (int k = 0; k < CF::PARTS; ++k) part[k][q] = next_part<CF::PARTS>(z0, z1);
-                                }
+                                for (int q = 0; q < 8; ++q) bad |= (e0 + q < p.Rg) ? (v[q] ^ phase) : 0u;
+                                if (!(bad & 1u)) break;
+                                if (poll.expired(ctrl, p, ST_Z)) break;
                             }
-                            uint8_t* o = zop + b * CF::ZB + (m >> 3) * 1024 + (m & 7) * 128 + ((pc ^ (m & 7)) << 4);
 #pragma unroll
-                            for (int k = 0; k < CF::PARTS; ++k)
-                                *reinterpret_cast<uint4*>(o + k * MMA_N * 128) = make_uint4(part[k][0], part[k][1], part[k][2], part[k][3]);
+                            for (int q = 0; q < 4; ++q) {
+                                float z0 = e0 + 2 * q < p.Rg ? unmark(v[2 * q]) : 0.f, z1 = e0 + 2 * q + 1 < p.Rg ? unmark(v[2 * q + 1]) : 0.f;
+#pragma unroll
+                                for (int k = 0; k < CF::PARTS; ++k) part[k][q] = next_part<CF::PARTS>(z0, z1);
+                            }
                         }
+                        uint8_t* o = zop + b * CF::ZB + (m >> 3) * 1024 + (m & 7) * 128 + ((pc ^ (m & 7)) << 4);
+#pragma unroll
+                        for (int k = 0; k < CF::PARTS; ++k)
+                            *reinterpret_cast<uint4*>(o + k * MMA_N * 128) = make_uint4(part[k][0], part[k][1], part[k][2], part[k][3]);
                     }
                     fence_proxy_async();
                     epi_sync();
