@@ -9,8 +9,9 @@
 //    from eight rows on, as a launch of its own in front it cost two grid hand-overs.
 //  * Expansion by MMAs: +-1.0 images of the U bits times z as a sum of bf16 parts, the parts side by side as ONE operand (an MMA
 //    costs 41 cycles at N = 16 and 50 at N = 64, so further parts are nearly free). Up to eight rows three parts, which
-//    are z itself, as the tile kernel's fp32 expansion has it (fp32 outputs 1.5e-7 off the 64-bit value, 2.4e-6 with two parts; 13.6 ->
-//    13.8 us at 8 rows); from nine rows two, which keep 2^-17 of it (2.5e-6). bf16 outputs are 1.66e-3 off either way.
+//    are z itself, as the tile kernel's fp32 expansion has it (fp32 outputs 1.1e-7 off the 64-bit value, 2.4e-6 with two parts); from
+//    nine rows two, which keep 2^-17 of it (2.5e-6). bf16 outputs are 1.66e-3 off either way. The chunks of a round are split
+//    into parts by all 256 threads at once: by one group of threads after the other 8 rows of 2560 -> 9728 took 15.2 us instead of 13.4.
 //  * A tile's contributors all add: contributor s of n takes words [s w / n, (s + 1) w / n) of the w that a partial sum has. With one finisher
 //    per tile the launch was as long as that CTA's n - 1 rounds of dependent loads after everybody else had left.
 //  * Nothing is announced, every hand-over is one memory round trip. Partial sums travel as 16-byte words [three rows' sums | launch count]
@@ -21,7 +22,7 @@
 //  * Scale factors are moved to TMEM by two groups of four warps in turn (one group's wait - load - store - arrive chain takes
 //    longer than a unit arrives at HBM speed), and the MMA warp waits on one barrier per unit.
 //
-// Measured (us per call, captured chain of distinct layers, K = N = 5120, r = 512, rows 8 / 16 / 32): 13.8 / 14.5 / 16.4 against
+// Measured (us per call, captured chain of distinct layers, K = N = 5120, r = 512, rows 8 / 16 / 32): 12.9 / 13.9 / 16.5 against
 // 20.4 / 24.4 / 29.9 with z on CUDA cores (8) or as a launch of its own (16, 32) and one finisher per tile.
 #pragma once
 #include "fused_cfg.cuh"

@@ -52,11 +52,10 @@ constexpr int ZR_MAX = 64;                       // ranks per chunk of the z sta
 constexpr int ZS_FIRST = 4;                      // U words per segment fetched ahead of the dependency wait
 // z is staged for the expansion in chunks of zs_words(ROWS) rank words (32 ranks each): ROWS x (32*words + 4) floats
 // (+4: rows start in different banks), at most ZS_BYTES.
-__host__ __device__ constexpr int zs_words(int rows) { return rows <= 8 ? 8 : 4; }
+__host__ __device__ constexpr int zs_words(int rows) { (void)rows; return 8; }      // (eight rows at most)
 __host__ __device__ constexpr int zs_stride(int rows) { return zs_words(rows) * 32 + 4; }
 constexpr int ZS_BYTES_SMALL = 8320;             // rows <= 8:  8 * 260 * 4
 constexpr int STAMP_WORDS = 16;                  // uint64 time stamps per CTA when debug stamps are on
-static_assert(32 * zs_stride(32) * 4 <= WORK_BYTES && 16 * zs_stride(16) * 4 <= WORK_BYTES, "z staging must fit in the work area");
 static_assert(8 * zs_stride(8) * 4 <= ZS_BYTES_SMALL && 4 * zs_stride(4) * 4 <= ZS_BYTES_SMALL, "z staging (rows <= 8)");
 constexpr int RED_OFF = ZS_BYTES_SMALL + 128;      // cluster mode (rows <= 8): partial sums of the peers start here,
 constexpr int RED_BYTES = WORK_BYTES - RED_OFF;    // after the z staging rows, [peer][row][128] floats

@@ -165,7 +165,10 @@ static bool consume_relayout_mark(cudaStream_t stream) {
     return true;
 }
 
-constexpr int BATCH_MIN_ROWS = 5;                 // activation rows from which schedules 2 and 4 are the batch kernel (batch_kernel.cuh)
+// Activation rows from which schedules 2 and 4 are the batch kernel (batch_kernel.cuh). Five is the first row count of the 8-row form
+// that no row-slab or cluster launch of one to four rows takes; below it the batch kernel has not been measured. (At four rows the
+// tile and cluster kernels take 16.9 / 16.0 us at 5120 x 5120, r = 512, the batch kernel 12.0 at five.)
+constexpr int BATCH_MIN_ROWS = 5;
 
 static int mma_n_for(int M) { return M <= 8 ? 8 : (M <= 16 ? 16 : 32); }
 
@@ -510,7 +513,7 @@ extern "C" int biloco_b200_schedule_info(int M, int N, int K, int R, int num_sms
     ScratchLayout L;
     if (!make_layout(M, N, K, R, num_sms, &L)) return BILOCO_ERR_SHAPE;
     out6[0] = L.ntile; out6[1] = L.nkt; out6[2] = L.G; out6[3] = L.max_slots; out6[4] = L.mma_n;
-    out6[5] = L.mma_n == 8 ? Cfg<8>::STAGES : (L.mma_n == 16 ? Cfg<16>::STAGES : Cfg<32>::STAGES);
+    out6[5] = M < BATCH_MIN_ROWS ? Cfg<8>::STAGES : (L.mma_n == 8 ? batch::Cfg<8>::RING : (L.mma_n == 16 ? batch::Cfg<16>::RING : batch::Cfg<32>::RING));
     return BILOCO_OK;
 }
 

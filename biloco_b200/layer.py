@@ -2,9 +2,9 @@
 
 Same constructor, ``quantize`` and ``forward`` signatures as the reference module (``biloco/layer.py:16-64``), but
 ``quantize`` keeps what the fused kernel streams — packed NVFP4 codes and block scales of the residual, bit-packed
-signs, bf16 coefficients — instead of dequantised bf16 copies, and ``forward`` is three enqueued device calls (the
-NVFP4 activation quantiser with the SmoothQuant division folded in, then the fused linear), with no host
-synchronisation. ``forward_fake_quant`` restates the reference's unfused bf16 forward on the same operands with
+signs, bf16 coefficients — instead of dequantised bf16 copies, and ``forward`` enqueues two launches up to 32 rows (the
+NVFP4 activation quantiser with the SmoothQuant division folded in, then the fused linear) and four above (maximum,
+quantiser, low-rank coefficients, GEMM), with no host synchronisation. ``forward_fake_quant`` restates the reference's unfused bf16 forward on the same operands with
 plain torch ops; the tests use it as the device-side comparator.
 """
 import ctypes

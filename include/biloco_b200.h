@@ -411,14 +411,14 @@ int biloco_b200_read_status(const void* scratch, int32_t* out16, biloco_stream_t
 /* Pipeline stages the fused kernel keeps in flight. 0 (default): chosen by the library - for M <= 8 with dependent
  * launch on, a ring of 4 stages so that two consecutive launches are resident on an SM at the same time (the second
  * one's first weights are in shared memory before the first has finished); otherwise all the stages that fit.
- * Other values are clamped to [4, what fits]. */
+ * Other values are clamped to [4, what fits]. Schedules 2 and 4 from five rows keep their own ring whatever is set. */
 #define BILOCO_OPT_RING 2
 /* Where a CTA of the fused kernel allows the next kernel of the stream to start (programmatic dependent launch):
  * -1 (default) chosen by the library, 0 after set-up, 4 after its dependency wait, 3 once its activation row has
- * landed, 1 after its z stage, 2 after its first expansion. Tuning aid. */
+ * landed, 1 after its z stage, 2 after its first expansion. Tuning aid. Schedules 2 and 4 from five rows: after set-up whatever is set. */
 #define BILOCO_OPT_TRIGGER 3
-/* Accepted without effect: from five activation rows the expansion of z through the U signs always runs on the tensor cores (bf16
- * sign image x z split into two bf16 parts, fp32 accumulation), below on the CUDA cores. */
+/* Accepted without effect: in schedules 2 and 4 from five activation rows the expansion of z through the U signs always runs on the
+ * tensor cores (bf16 sign image x z split into two or three bf16 parts, fp32 accumulation), below on the CUDA cores. */
 #define BILOCO_OPT_LR_TC 4
 /* Budget of a device-side wait in microseconds (default 200 000; <= 0 restores the default). A wait that runs out
  * records its code in the status words and the launch returns (row-slab schedule, schedules 2 and 4 from five rows, prompt forward; the other launches keep 200 ms).
@@ -435,7 +435,8 @@ int biloco_b200_read_status(const void* scratch, int32_t* out16, biloco_stream_t
 #define BILOCO_OPT_ZTC 8
 int biloco_b200_set_option(int option, int value);
 
-/* Debug aid: while a device buffer is registered here, every fused launch of this process writes 16 uint64
+/* Debug aid: while a device buffer is registered here, every fused launch of this process (but for schedules 2 and 4 from five
+ * rows) writes 16 uint64
  * %globaltimer stamps per CTA into it (CTA c at words 16c..16c+15: 0 set-up done, 1 z published, 2 z complete seen,
  * 3 expansion done, 4 accumulators ready, 5/6 first/last segment stored, 7 last stage consumed, 8 first z reads
  * landed, 9 z computed, 10 CTA entry, 11 previous kernel complete, 13 CTA exit). bytes >= 128 * CTAs; a larger

@@ -608,33 +608,31 @@ def test_batch_partial_sums_are_whole(kernel, M, K, N):
 @pytest.mark.parametrize("M,K,N,R,mode", [(32, 5120, 5120, 512, 2), (16, 5120, 5120, 512, 2), (32, 1024, 1024, 128, 2), (32, 2560, 1024, 200, 2),
                                           (24, 256, 640, 72, 2), (32, 5120, 2560, 1024, 2), (8, 5120, 5120, 512, 5), (4, 2048, 1024, 64, 2),
                                           (17, 8192, 1024, 512, 2)])
-def test_fused_with_tensor_core_z_launch(kernel, lib, M, K, N, R, mode):
-    """The z stage as a tensor-core launch of its own in front of the fused launch (default from 16 rows; forced here for
-    the smaller batches): against the oracle's unfused value with non-zero block scales, bit-identical call after call and
-    within an ulp-level distance of the in-kernel CUDA-core z stage (same sums, other order of additions). Ranks that are
-    not a multiple of 128, a K of four chunks, eight rank blocks."""
-    from biloco_b200 import _lib
+def test_fused_at_many_rows_and_ragged_ranks(kernel, lib, M, K, N, R, mode):
+    """Larger batches against the oracle's unfused value with non-zero block scales, bit-identical call after call: ranks that are not a
+    multiple of 128, a K of four chunks, eight rank blocks; and, where the schedule computes z and expands it on the tensor cores (mode 2
+    from five rows), the same shape one row at a time on schedules that do both on CUDA cores: an ulp-level distance (same
+    sums, other order of additions, z as two or three bf16 parts)."""
     if mode not in kernel.supported_modes(M, N, K, R):
         pytest.skip("schedule not available for this shape")
     p = orc.random_problem(M, K, N, R, scales="random", seed=300 + M + R)
     t = dev_problem(p)
     y_ref, _ = oracle_outputs(p, M)
-    outs = {}
-    try:
-        for ztc in (1, 0):
-            assert lib.biloco_b200_set_option(_lib.OPT_ZTC, ztc) == 0
-            g = kernel.BiLoCoGemm(t["W"], t["W_sf"], t["alpha"], t["V_packed"], t["U_packed"], t["S"], M=M, mode=mode)
-            ys = []
-            for _ in range(4):
-                ys.append(g(t["A_pad"], t["A_sf"], t["X"]).view(-1, N)[:M].clone())
-            torch.cuda.synchronize()
-            assert g.status()[0] == 0, g.status()[:4]
-            assert all(torch.equal(ys[0].view(torch.int16), y.view(torch.int16)) for y in ys[1:])
-            check_against_unfused(ys[0].float().cpu().numpy(), y_ref, f"ztc={ztc}")
-            outs[ztc] = ys[0].float()
-    finally:
-        lib.biloco_b200_set_option(_lib.OPT_ZTC, -1)
-    assert float((outs[1] - outs[0]).abs().max()) <= 2.0 ** -7 * float(outs[0].abs().max())      # (bf16 outputs: at most an ulp apart)
+    g = kernel.BiLoCoGemm(t["W"], t["W_sf"], t["alpha"], t["V_packed"], t["U_packed"], t["S"], M=M, mode=mode)
+    ys = []
+    for _ in range(4):
+        ys.append(g(t["A_pad"], t["A_sf"], t["X"]).view(-1, N)[:M].clone())
+    torch.cuda.synchronize()
+    assert g.status()[0] == 0, g.status()[:4]
+    assert all(torch.equal(ys[0].view(torch.int16), y.view(torch.int16)) for y in ys[1:])
+    check_against_unfused(ys[0].float().cpu().numpy(), y_ref, f"mode {mode}")
+    if mode == 2 and M >= 5:
+        from biloco_b200 import fp4
+        one = kernel.BiLoCoGemm(t["W"], t["W_sf"], t["alpha"], t["V_packed"], t["U_packed"], t["S"], M=1, mode=2)
+        sf = fp4.unswizzle_scales(t["A_sf"], M, K)
+        for m in (0, M // 2, M - 1):
+            y1 = one(t["A_pad"][:, m:m + 1].contiguous(), fp4.swizzle_scales(sf[m:m + 1]), t["X"][m:m + 1].contiguous()).view(-1, N)[0].float()
+            assert float((ys[0][m].float() - y1).abs().max()) <= 2.0 ** -7 * float(y1.abs().max())      # (bf16 outputs: at most an ulp apart)
 
 
 @pytest.mark.parametrize("M,mode", [(1, 5), (1, 2), (8, 5), (32, 2)])

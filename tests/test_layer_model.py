@@ -151,9 +151,9 @@ def test_config0_layer(M):
 
 @pytest.mark.gpu
 def test_long_input_shares_one_tensor_scale_and_smoothed_follows_the_buffers():
-    """More than 32 rows go through the kernel in blocks of 32 that all use ONE NVFP4 tensor scale, taken over the whole
-    smoothed activation as the reference does (biloco/fp4.py:3-4): with one block 50x larger than the rest, per-block
-    scales would quantise the small rows far more finely than the fake-quant forward does. And a layer whose buffers
+    """More than 32 rows go through the prompt kernels, which use ONE NVFP4 tensor scale for all of them, taken over the whole
+    smoothed activation as the reference does (biloco/fp4.py:3-4): with 32 rows 50x larger than the rest, scales of their
+    own would quantise the small rows far more finely than the fake-quant forward does. And a layer whose buffers
     are filled by load_state_dict divides by its smoothing vector like the layer that was saved."""
     torch.manual_seed(3)
     bl = BiLoCoLinear.synthetic(1024, 512, 64, "cuda", seed=5)
