@@ -23,10 +23,10 @@ IMPLEMENTED_MODES = (2, 4, 5, 7)
 
 # Time per call of every implemented mode per (M, rank) on B200 at K = N = 5120, HBM-cold, from `bench.py --table` (us;
 # mode 2 / mode 5 / mode 7 where the mode takes the point; M >= 8: mode 2, from five rows the batch kernel; mode 5 took 14.7 / 16.5 / 20.4 / 31.3 at M = 8):
-#   r = 128 : M=1 11.3/9.6/8.5    M=2 12.0/9.7/8.5    M=4 12.9/12.7/10.5  M=8 11.0  M=16 12.6  M=32 15.5
-#   r = 256 : M=1 11.9/9.8/8.2    M=2 12.7/10.1/8.6   M=4 14.6/14.4/10.4  M=8 11.9  M=16 12.9  M=32 15.8
-#   r = 512 : M=1 12.7/10.2/8.9   M=2 14.7/12.6/9.4   M=4 16.9/16.0/10.7  M=8 13.5  M=16 14.6  M=32 17.4
-#   r = 1024: M=1 14.9/14.1/10.2  M=2 17.6/18.5/12.4  M=4 21.6/21.5       M=8 18.1  M=16 19.6  M=32 23.2
+#   r = 128 : M=1 11.3/9.6/8.5    M=2 12.0/9.7/8.5    M=4 12.9/12.7/10.5  M=8 11.3  M=16 12.3  M=32 14.7
+#   r = 256 : M=1 11.9/9.8/8.2    M=2 12.7/10.1/8.6   M=4 14.6/14.4/10.4  M=8 11.8  M=16 12.9  M=32 14.9
+#   r = 512 : M=1 12.7/10.2/8.9   M=2 14.7/12.6/9.4   M=4 16.9/16.0/10.7  M=8 12.9  M=16 13.9  M=32 16.4
+#   r = 1024: M=1 14.9/14.1/10.2  M=2 17.6/18.5/12.4  M=4 21.6/21.5       M=8 15.9  M=16 17.6  M=32 21.2
 # Mode 5 does not take M > 8, mode 7 not M > 4 (nor r = 1024 at M = 4); mode 4 loses everywhere. Ranks below 128 were not
 # measured and follow r = 128. DEFAULT_MODE is the table WITHOUT mode 7 (what a stream with other kernels between the linears
 # uses: with a quantiser in front of every linear mode 7 wins a captured chain of small layers, 12.9 -> 11.2 us at 4096 x 2560 and
